@@ -200,3 +200,44 @@ def tolerance(case):
     2-norm 0.006 .. 0.015 for 288 .. 8771 tokens, largest difference 0.04 .. 0.12 of the result's
     root mean square, 0.23 in the first rows of a causal call."""
     return {"rel": 0.03, "max": 0.5}
+
+
+def _attend64(q, k, v, causal):
+    """(softmax(q k^T / sqrt(d)) v, log-sum-exp) of one head in 64 bits, a block of queries at a time."""
+    n, m = q.shape[0], k.shape[0]
+    out = torch.empty((n, v.shape[1]), dtype=torch.float64, device=q.device)
+    lse = torch.empty((n,), dtype=torch.float64, device=q.device)
+    k, v = k.double(), v.double()
+    keys = torch.arange(m, device=q.device)
+    for i in range(0, n, 4096):
+        s = (q[i:i + 4096].double() @ k.T) * q.shape[1] ** -0.5
+        if causal:
+            s.masked_fill_(keys[None, :] > torch.arange(i, i + s.shape[0], device=q.device)[:, None], -math.inf)
+        lse[i:i + 4096] = torch.logsumexp(s, 1)
+        out[i:i + 4096] = torch.exp_(s.sub_(lse[i:i + 4096, None])) @ v
+    return out, lse
+
+
+def exact(case, seed):
+    """Plain attention in 64 bits.  None where e4m3 score codes meet keys scaled x50: the format alone
+    puts such outputs 0.2 off, so the distance says nothing about an implementation."""
+    if case["dominant"] > 0 and (case["e4m3"] or case["dtype"] == "bf16"):
+        return None
+    state = prepare(case, seed)
+    q, k, v = state["q"], state["k"], state["v"]
+    group = case["hq"] // case["hkv"]
+    if case["kind"] == "packed":
+        out = torch.zeros(q.shape, dtype=torch.float64, device=q.device)
+        cu = state["cu"].tolist()
+        for a, z in zip(cu, cu[1:]):
+            for h in range(case["hq"]):
+                out[a:z, h] = _attend64(q[a:z, h], k[a:z, h // group], v[a:z, h // group], case["causal"])[0]
+        return out
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    heads = (lambda t: t) if case["layout"] == "HND" else (lambda t: t.transpose(1, 2))
+    lse = torch.empty((case["b"], case["hq"], case["nq"]), dtype=torch.float64, device=q.device)
+    for b in range(case["b"]):
+        for h in range(case["hq"]):
+            o, lse[b, h] = _attend64(heads(q)[b, h], heads(k)[b, h // group], heads(v)[b, h // group], case["causal"])
+            heads(out)[b, h] = o
+    return (out, lse) if case["lse"] else out
