@@ -59,6 +59,7 @@
 // TMEM, and CTAs that start later return at once.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "sage_common.cuh"
@@ -295,6 +296,12 @@ struct AttnKArgs {
   float skip_log2;    // FAST kernels: key tiles whose scores all lie this far (exponent domain) below the running maxima are not exponentiated
   unsigned* skipped;  // FAST kernels, optional: receives the number of (warp, key tile) pairs that were skipped
   int32_t* status;
+  int rows_per_head;  // query rows of one head: Nq, unless grouped heads are folded into one unit (see launch_attention)
+  int heads_per_unit; // heads folded into one unit (1: none)
+  int splits, split_tiles;  // SPLIT kernels: shares of the key range, key tiles in a share
+  float* part_o;      // SPLIT kernels: (splits, units x rows, 128) unnormalised output rows
+  float2* part_ml;    // SPLIT kernels: (splits, units x rows) {c_q * m, l}
+  float* part_max;    // SPLIT kernels: (splits, units x rows) largest score of the share, in the u domain
   const int *cu_q, *cu_k;   // VARLEN kernels: cumulative token counts of the packed batch (B + 1 entries each)
   long long Tq, Tk;         // VARLEN kernels: tokens in the packed q / out and k / v tensors
 };
@@ -317,11 +324,21 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
 // operands, the grid is sized for the longest sequence allowed; each sequence's own lengths and the
 // first row of its output come from cu_q / cu_k, and a CTA whose query tile lies past its
 // sequence's end returns at once.
-template <bool INT8, bool CAUSAL, typename OutT, int NQ, bool FAST, bool VARLEN>
+// SPLIT: a share of the key range per CTA (blockIdx.x = query tile * splits + share), in two launches.
+// SPLIT_MAX only finds each row's score maximum in the share (part_max).  SPLIT_SUM starts from the
+// maximum over the shares before its own, so that its running maxima, and with them the e4m3 codes of
+// P, are those of one walk over all keys; it leaves its unnormalised output rows, maxima and sums in
+// part_o / part_ml, and combine_splits_kernel merges them.  (Shares with maxima of their own round P
+// elsewhere: 0.035 of the result's 2-norm away from the unsplit kernel, as far as e4m3 goes.)
+// RAGGED and both of these also fold grouped heads and leave out softmax warps without a row; the
+// kernels without either (WHOLE) carry none of that code: it costs their schedule 1 to 6 %.
+enum { WHOLE = 0, RAGGED = 1, SPLIT_MAX = 2, SPLIT_SUM = 3 };
+template <bool INT8, bool CAUSAL, typename OutT, int NQ, bool FAST, bool VARLEN, int ROWS>
 __global__ void __launch_bounds__(Shape<NQ>::THREADS, Shape<NQ>::CTAS_PER_SM)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const AttnKArgs a) {
   using L = Shape<NQ>;
+  constexpr bool SPLIT = ROWS == SPLIT_MAX || ROWS == SPLIT_SUM;
   constexpr uint32_t OFF_Q = L::OFF_Q, OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_P = L::OFF_P, OFF_SK = L::OFF_SK,
                      OFF_SV = L::OFF_SV, OFF_BAR = L::OFF_BAR, OFF_MISC = L::OFF_MISC;
   extern __shared__ uint8_t smem_raw[];
@@ -336,7 +353,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // first query tile of this CTA (causal: longest first); softmax group g owns tile q_tile0 + g
-  const int q_tile0 = NQ * (CAUSAL ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x);
+  const int q_tile0 = NQ * (CAUSAL ? (int)(gridDim.x - 1 - blockIdx.x)
+                                   : SPLIT ? (int)blockIdx.x / a.splits : (int)blockIdx.x);
+  const int share = SPLIT ? (int)blockIdx.x % a.splits : 0;
+  const int k_tile0 = SPLIT ? share * a.split_tiles : 0;     // first key tile of this CTA
   const int bh = blockIdx.y;                          // (batch, query head)
   const int bh_kv = (int)((bh / a.Hq) * a.H + (bh % a.Hq) / a.group);   // its (batch, K/V head)
   // Key tiles query tile g visits: all of them, or when causal those up to its diagonal (a causal
@@ -361,7 +381,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       return;
     }
   }
-  const int key_tiles = VARLEN ? (int)((Nk_live + TILE - 1) / TILE) : (int)(a.N_pad / TILE);
+  const int key_tiles = VARLEN ? (int)((Nk_live + TILE - 1) / TILE)
+                        : SPLIT ? min((int)(a.N_pad / TILE) - k_tile0, a.split_tiles) : (int)(a.N_pad / TILE);
+  if (SPLIT) Nk_live = a.N - (long long)k_tile0 * TILE;      // keys from the first one of this share on
+  // Softmax warps of query tile g that hold a row that exists (16 rows each; one at least, so that
+  // an empty second tile keeps its barriers turning).  The others stay out of the loop and of the
+  // barriers' counts: their rows of P are never written and their rows of O never read.
+  auto live_warps = [&](int g) {
+    if (ROWS == WHOLE) return 8;
+    const long long rows = (VARLEN ? Nq_live : a.Nq) - (long long)(q_tile0 + g) * TILE;
+    return (int)min(max((rows + 15) / 16, 1LL), 8LL);
+  };
   auto tiles_of = [&](int g) { return CAUSAL ? min(q_tile0 + g + 1, key_tiles) : key_tiles; };
   const int n_load = tiles_of(NQ - 1);
 
@@ -375,8 +405,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     for (int g = 0; g < NQ; ++g) {
       mbar_init(bar(BAR_SF + BAR_PER_TILE * g), 1);
-      mbar_init(bar(BAR_SFREE + BAR_PER_TILE * g), 8);
-      mbar_init(bar(BAR_PF + BAR_PER_TILE * g), 8);
+      mbar_init(bar(BAR_SFREE + BAR_PER_TILE * g), (uint32_t)live_warps(g));
+      mbar_init(bar(BAR_PF + BAR_PER_TILE * g), (uint32_t)live_warps(g));
       mbar_init(bar(BAR_PV + BAR_PER_TILE * g), 1);
     }
     misc[1] = (*reinterpret_cast<volatile int32_t*>(a.status) != 0) ? 1u : 0u;
@@ -414,6 +444,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (lane == 0) {
         const int g = warp & 1, gb = BAR_PER_TILE * g;
         const int n_tiles = tiles_of(g);
+        const uint32_t n_live = FAST ? (uint32_t)live_warps(g) : 0u;
         bool ok = true;
         if (warp < 2) {
           // ------------------------------- Q.K^T issuers ---------------------------
@@ -477,7 +508,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               volatile uint32_t* cnt = misc + 4 + 2 * g + (jj & 1);
               const uint32_t c8 = *cnt;
               if (c8 != 0u) *cnt = 0u;
-              all_zero = (c8 == 8u);
+              all_zero = (c8 == n_live);
             }
             tc_fence_after();
             if (!all_zero)
@@ -500,8 +531,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         mbar_expect_tx(bar(BAR_Q), NQ * TILE_BYTES);
         for (int g = 0; g < NQ; ++g)                          // rows past the last query arrive as zeros
           tma_load_3d(base + OFF_Q + g * TILE_BYTES, &tm_q, bar(BAR_Q), 0, (q_tile0 + g) * TILE, bh);
-        const float* sk_row = a.sk + (size_t)bh_kv * a.N_pad;
-        const float* sv_row = a.svp + (size_t)bh_kv * a.N_pad;
+        const float* sk_row = a.sk + (size_t)bh_kv * a.N_pad + (size_t)k_tile0 * TILE;
+        const float* sv_row = a.svp + (size_t)bh_kv * a.N_pad + (size_t)k_tile0 * TILE;
         auto load_k = [&](int j) -> bool {
           const int s = j & 1;
           const uint32_t par = ((uint32_t)(j >> 1) & 1u) ^ 1u;
@@ -509,7 +540,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           // The tile's scale rows ride on the K barrier into a 4-slot ring: slot j&3 is rewritten
           // only after QK(j+2) has completed, which needs every softmax warp to be past tile j.
           mbar_expect_tx(bar(BAR_KF + s), TILE_BYTES + 2 * VEC_BYTES);
-          tma_load_3d(base + OFF_K + s * TILE_BYTES, &tm_k, bar(BAR_KF + s), 0, j * TILE, bh_kv);
+          tma_load_3d(base + OFF_K + s * TILE_BYTES, &tm_k, bar(BAR_KF + s), 0, (k_tile0 + j) * TILE, bh_kv);
           bulk_load(base + OFF_SK + (j & 3) * VEC_BYTES, sk_row + (size_t)j * TILE, VEC_BYTES, bar(BAR_KF + s));
           bulk_load(base + OFF_SV + (j & 3) * VEC_BYTES, sv_row + (size_t)j * TILE, VEC_BYTES, bar(BAR_KF + s));
           return true;
@@ -518,11 +549,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int j = 0; ok && j < L::K_AHEAD && j < n_load; ++j) ok = load_k(j);
         for (int j = 0; ok && j < n_load; ++j) {
           if (j + L::K_AHEAD < n_load && !load_k(j + L::K_AHEAD)) break;
+          if (ROWS == SPLIT_MAX) continue;                   // no P.V
           const int sv = j % L::V_STAGES;
           const uint32_t parv = ((uint32_t)(j / L::V_STAGES) & 1u) ^ 1u;
           if (!mbar_wait(bar(BAR_VE + sv), parv, cta_abort, a.status, ST_TIMEOUT_PRODUCER)) break;
           mbar_expect_tx(bar(BAR_VF + sv), TILE_BYTES);
-          tma_load_3d(base + OFF_V + sv * TILE_BYTES, &tm_v, bar(BAR_VF + sv), j * TILE, 0, bh_kv);
+          tma_load_3d(base + OFF_V + sv * TILE_BYTES, &tm_v, bar(BAR_VF + sv), (k_tile0 + j) * TILE, 0, bh_kv);
         }
       }
     } else if (warp == 1) {
@@ -530,6 +562,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int g = 0;
       const int gb = BAR_PER_TILE * g;
       const int n_tiles = tiles_of(g);
+      const uint32_t n_live = FAST ? (uint32_t)live_warps(g) : 0u;
       if (lane == 0) {
         constexpr uint32_t IDESC_QK = INT8 ? IDESC_I8 : IDESC_F8;
         bool ok = mbar_wait(bar(BAR_Q), 0, cta_abort, a.status, ST_TIMEOUT_MMA);
@@ -547,13 +580,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             tc_commit(bar(BAR_KE + s));
             tc_commit(bar(BAR_SF + gb));
           }
-          if (j > 0) {
+          if (ROWS != SPLIT_MAX && j > 0) {
             const int jj = j - 1, s = jj % L::V_STAGES;
             ok = mbar_wait(bar(BAR_VF + s), (uint32_t)(jj / L::V_STAGES) & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
             if (ok) ok = mbar_wait(bar(BAR_PF + gb), (uint32_t)jj & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
             if (!ok) break;
             // FAST kernels: a warp that skips a tile counts itself before it arrives at the P
-            // barrier.  When all eight warps of the query tile did, P(jj) is all zeros and the
+            // barrier.  When all live warps of the query tile did, P(jj) is all zeros and the
             // product is not issued; the two commits still release the V stage and complete the
             // P.V barrier (the first tile is never skipped, so the accumulator is initialised).
             bool all_zero = false;
@@ -561,7 +594,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               volatile uint32_t* cnt = misc + 4 + 2 * g + (jj & 1);
               const uint32_t c8 = *cnt;
               if (c8 != 0u) *cnt = 0u;
-              all_zero = (c8 == 8u);
+              all_zero = (c8 == n_live);
             }
             tc_fence_after();
             if (!all_zero)
@@ -588,11 +621,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int g = (NQ == 1) ? 0 : (warp - 4) >> 3;        // which query tile of the CTA
       const int gb = BAR_PER_TILE * g;
       const int q_tile = q_tile0 + g;
-      const int n_tiles = tiles_of(g);
       const int quarter = warp & 3;                         // TMEM lane quarter this warp may touch
       const int sub = ((warp - 4) >> 2) & 1;                // which 16 lanes of the quarter
       const int r0 = lane >> 2, c = lane & 3;
       const int lane_base = 32 * quarter + 16 * sub;
+      if (ROWS == WHOLE || lane_base < 16 * live_warps(g)) {
+      const int n_tiles = tiles_of(g);
       const int rowA = lane_base + r0, rowB = rowA + 8;     // this thread's two query rows of the tile
       const long long q_rowA = (long long)q_tile * TILE + rowA, q_rowB = q_rowA + 8;
       const uint32_t t_s = tmem + ((uint32_t)lane_base << 16) + L::tmem_s(g);
@@ -603,6 +637,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const float cqB = (q_rowB < (VARLEN ? Nq_live : a.Nq)) ? __fmul_rn(sl2, __ldg(a.sq + (size_t)bh * a.Nq + q_rowB)) : 1.f;
       const float2 cqA2 = make_float2(cqA, cqA), cqB2 = make_float2(cqB, cqB);
       float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;
+      if (ROWS == SPLIT_SUM) {
+        const size_t rows = (size_t)gridDim.y * a.Nq, row0 = (size_t)bh * a.Nq;
+        for (int s = 0; s < share; ++s) {
+          if (q_rowA < a.Nq) mA = fmaxf(mA, a.part_max[s * rows + row0 + q_rowA]);
+          if (q_rowB < a.Nq) mB = fmaxf(mB, a.part_max[s * rows + row0 + q_rowB]);
+        }
+      }
       bool ok = true;
       // P tile: 16 keys of row r (chunk m) at (r / 8) * 1024 + m * 128 + (r % 8) * 16, so that the
       // eight stores of a row differ by a constant and a warp's store covers 128 contiguous bytes
@@ -752,8 +793,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
           }
         } else {
-          if ((long long)(j + 1) * TILE > (VARLEN ? Nk_live : a.N)) {
-            const int live = (int)((VARLEN ? Nk_live : a.N) - (long long)j * TILE);   // tile-local key >= live is masked
+          if ((long long)(j + 1) * TILE > (VARLEN || SPLIT ? Nk_live : a.N)) {
+            const int live = (int)((VARLEN || SPLIT ? Nk_live : a.N) - (long long)j * TILE);   // tile-local key >= live is masked
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const int key = 16 * (i >> 1) + 4 * c + 2 * (i & 1);
@@ -779,6 +820,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
         mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2));
         const float mA_new = fmaxf(mA, mxA), mB_new = fmaxf(mB, mxB);
+        if (ROWS == SPLIT_MAX) { mA = mA_new; mB = mB_new; continue; }
         const float mA_use = (mA_new == -INFINITY) ? 0.f : mA_new;
         const float mB_use = (mB_new == -INFINITY) ? 0.f : mB_new;
         float alphaA, alphaB;
@@ -873,6 +915,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (FAST && a.skipped != nullptr && lane == 0 && n_skipped > 0) atomicAdd(a.skipped, (unsigned)n_skipped);
 
       // ------------------------------- epilogue -----------------------------------
+      if (ROWS == SPLIT_MAX) {
+        const size_t row0 = (size_t)share * gridDim.y * a.Nq + (size_t)bh * a.Nq;
+        if (ok && c == 0 && q_rowA < a.Nq) a.part_max[row0 + q_rowA] = mA;
+        if (ok && c == 0 && q_rowB < a.Nq) a.part_max[row0 + q_rowB] = mB;
+        ok = false;
+      }
       if (ok) {
         ok = mbar_wait(bar(BAR_PV + gb), (uint32_t)(n_tiles - 1) & 1u, cta_abort, a.status, ST_TIMEOUT_SOFTMAX);
         ok = __all_sync(0xffffffffu, ok);
@@ -882,6 +930,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // total row sums: the four quarters were scaled with the same running maximum
         lA += __shfl_xor_sync(0xffffffffu, lA, 1); lB += __shfl_xor_sync(0xffffffffu, lB, 1);
         lA += __shfl_xor_sync(0xffffffffu, lA, 2); lB += __shfl_xor_sync(0xffffffffu, lB, 2);
+        if constexpr (ROWS == SPLIT_SUM) {
+          const size_t row0 = (size_t)share * gridDim.y * a.Nq + (size_t)bh * a.Nq;
+          if (c == 0) {
+            if (q_rowA < a.Nq) a.part_ml[row0 + q_rowA] = make_float2(cqA * mA, lA);
+            if (q_rowB < a.Nq) a.part_ml[row0 + q_rowB] = make_float2(cqB * mB, lB);
+          }
+          float* oA = a.part_o + (row0 + q_rowA) * HD + 2 * c;
+          uint32_t o[64];
+          tmem_ld_16x256b_x16(t_o, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            if (q_rowA < a.Nq) *reinterpret_cast<uint2*>(oA + 8 * i) = make_uint2(o[4 * i + 0], o[4 * i + 1]);
+            if (q_rowB < a.Nq) *reinterpret_cast<uint2*>(oA + 8 * HD + 8 * i) = make_uint2(o[4 * i + 2], o[4 * i + 3]);
+          }
+        } else {
         const float S = __ldg(a.s_fold + bh_kv);
         const float invA = (lA > 0.f) ? __fdiv_rn(S, __fmul_rn(lA, F8_MAX)) : 0.f;
         const float invB = (lB > 0.f) ? __fdiv_rn(S, __fmul_rn(lB, F8_MAX)) : 0.f;
@@ -901,6 +965,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         OutT* orowA = reinterpret_cast<OutT*>(a.out) + (VARLEN ? o_first : b * a.o_sb) + h * a.o_sh + q_rowA * a.o_sr + 2 * c;
         OutT* orowB = orowA + 8 * a.o_sr;
+        if (ROWS == RAGGED && a.heads_per_unit > 1) {   // rows of a folded unit: heads_per_unit heads of rows_per_head rows
+          const long long o_unit = b * a.o_sb + h * a.heads_per_unit * a.o_sh + 2 * c;
+          const unsigned hA = (unsigned)q_rowA / (unsigned)a.rows_per_head, hB = (unsigned)q_rowB / (unsigned)a.rows_per_head;
+          orowA = reinterpret_cast<OutT*>(a.out) + o_unit + hA * a.o_sh + (q_rowA - (long long)hA * a.rows_per_head) * a.o_sr;
+          orowB = reinterpret_cast<OutT*>(a.out) + o_unit + hB * a.o_sh + (q_rowB - (long long)hB * a.rows_per_head) * a.o_sr;
+        }
         const float* vm = (a.vmean != nullptr) ? a.vmean + (size_t)bh_kv * HD + 2 * c : nullptr;
         uint32_t o[64];
         tmem_ld_16x256b_x16(t_o, o);
@@ -918,6 +988,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (q_rowB < (VARLEN ? Nq_live : a.Nq)) *reinterpret_cast<uint32_t*>(orowB + 8 * i) = pack2<OutT>(fb0, fb1);
           }
         }
+        }
+      }
       }
     }
   }
@@ -934,6 +1006,53 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Merges the shares of a SPLIT call: out = sum_s 2^(m_s - M) O_s * (S_fold / (L * 448)) with M the
+// largest share maximum and L = sum_s 2^(m_s - M) l_s, all in fp32; one warp per query row, four
+// channels per lane.  Reads splits x 520 bytes per row, which the shares have just written (L2).
+// ------------------------------------------------------------------------------------------------
+template <typename OutT>
+__global__ void __launch_bounds__(256) combine_splits_kernel(const AttnKArgs a, long long rows) {
+  wait_for_predecessor();
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= rows || *reinterpret_cast<volatile int32_t*>(a.status) != 0) return;
+  float M = -INFINITY;
+  for (int s = 0; s < a.splits; ++s) M = fmaxf(M, a.part_ml[s * rows + r].x);
+  const float M_use = (M == -INFINITY) ? 0.f : M;
+  float l = 0.f;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int s = 0; s < a.splits; ++s) {
+    const float2 ml = a.part_ml[s * rows + r];
+    const float4 p = reinterpret_cast<const float4*>(a.part_o + (s * rows + r) * HD)[lane];
+    const float w = ex2(ml.x - M_use);
+    l = __fmaf_rn(w, ml.y, l);
+    o.x = __fmaf_rn(w, p.x, o.x); o.y = __fmaf_rn(w, p.y, o.y);
+    o.z = __fmaf_rn(w, p.z, o.z); o.w = __fmaf_rn(w, p.w, o.w);
+  }
+  const long long unit = r / a.Nq, row = r - unit * a.Nq;             // unit = (batch, K/V head) when heads are folded
+  const long long b = unit / a.Hq, h = unit - b * a.Hq;
+  const long long bh_kv = b * a.H + h / a.group;
+  const float inv = (l > 0.f) ? __fdiv_rn(__ldg(a.s_fold + bh_kv), __fmul_rn(l, F8_MAX)) : 0.f;
+  if (a.lse != nullptr && lane == 0) {
+    float v = (l > 0.f) ? 0.6931471805599453f * (M_use + log2f(l)) : -INFINITY;
+    if (a.qm != nullptr) v += a.sm_scale * __ldg(a.qm + r);
+    a.lse[r] = v;
+  }
+  if (4 * lane < a.D) {
+    float4 f = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
+    if (a.vmean != nullptr) {
+      const float4 mu = __ldg(reinterpret_cast<const float4*>(a.vmean + bh_kv * HD) + lane);
+      f.x += mu.x; f.y += mu.y; f.z += mu.z; f.w += mu.w;
+    }
+    const long long hh = row / a.rows_per_head;
+    OutT* dst = reinterpret_cast<OutT*>(a.out) + b * a.o_sb + (h * a.heads_per_unit + hh) * a.o_sh +
+                (row - hh * a.rows_per_head) * a.o_sr + 4 * lane;
+    *reinterpret_cast<uint2*>(dst) = make_uint2(pack2<OutT>(f.x, f.y), pack2<OutT>(f.z, f.w));
   }
 }
 
@@ -982,10 +1101,10 @@ constexpr float SKIP_LOG2_DEFAULT = 40.f;
 static std::atomic<float> g_skip_log2{SKIP_LOG2_DEFAULT};
 void set_skip_log2(float t) { g_skip_log2.store(t < 0.f ? SKIP_LOG2_DEFAULT : t, std::memory_order_relaxed); }
 
-template <bool INT8, bool CAUSAL, typename OutT, int NQ, bool FAST, bool VARLEN = false>
+template <bool INT8, bool CAUSAL, typename OutT, int NQ, bool FAST, bool VARLEN = false, int ROWS = WHOLE>
 static cudaError_t launch_inst(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                const AttnKArgs& ka, dim3 grid, cudaStream_t st) {
-  auto kern = attn_fwd_kernel<INT8, CAUSAL, OutT, NQ, FAST, VARLEN>;
+  auto kern = attn_fwd_kernel<INT8, CAUSAL, OutT, NQ, FAST, VARLEN, ROWS>;
   using L = Shape<NQ>;
   // the opt-in to more than 48 KB of dynamic shared memory is per device and per instantiation;
   // it is made once (short calls are dominated by host-side work)
@@ -1025,7 +1144,65 @@ int choose_tiles_per_cta(int64_t q_tiles, int64_t bhq, bool causal, int sms) {
   return rounds_two <= rounds_one ? 2 : 1;
 }
 
-cudaError_t launch_attention(const AttnParams& p, cudaStream_t st, const char** why) {
+// Into how many shares the keys of a call with few queries are split.  Such a call has fewer
+// one-tile CTAs than the GPU has SMs, each walking all keys alone; shares of at least eight key
+// tiles are handed out until there are two CTAs per SM.  The bound of 128 queries a head keeps
+// longer calls, whose key tiles the negligible-tile tests may drop, on one pass.  2 x 8 K/V heads x
+// 4 x 4 query rows x 16 384 keys: 64 CTAs of 128 key tiles took 182 us, 256 of 8 with both passes
+// and the merge 35 us (whole call 267 -> 118 us).
+int key_splits(int64_t B, int64_t Hq, int64_t H, int64_t Nq, int64_t Nk, int sms) {
+  const int64_t key_tiles = (Nk + TILE - 1) / TILE;
+  const int64_t units = B * H * ((Nq * (Hq / H) + TILE - 1) / TILE);
+  if (Nq > TILE || key_tiles < 16 || units >= sms) return 1;
+  return (int)std::min<int64_t>(2 * sms / units, key_tiles / 8);
+}
+size_t split_scratch_bytes(int64_t B, int64_t Hq, int64_t H, int64_t Nq, int64_t Nk) {
+  const int n = key_splits(B, Hq, H, Nq, Nk, SPLIT_SIZING_SMS);
+  return n < 2 ? 0 : (size_t)n * (size_t)(B * Hq * Nq) * (HD + 3) * sizeof(float);
+}
+
+// Calls whose last query tiles are mostly empty take the RAGGED kernels: grouped query heads are
+// folded into their K/V head's unit (a unit's Hq/H heads x Nq rows are consecutive rows of Q8 and
+// SQ anyway, a row's result does not depend on its place in a tile, and only the epilogue needs to
+// know where a row belongs), and softmax warps without a row stay idle.  Taken when that leaves
+// out a tenth of the softmax warps or more (48 x 288 x 288: 12.7 -> 11.4 us); full tiles lose 1 to
+// 2 % in those kernels (48 x 4 096 x 4 096: 391 -> 396 us).
+static bool mostly_empty_tiles(const AttnParams& p) {
+  const int64_t rows = p.Nq * (p.Hq / p.H);
+  const int64_t warps = 8 * p.Hq * ((p.Nq + TILE - 1) / TILE), live = p.H * ((rows + 15) / 16);
+  return rows <= ((int64_t)1 << 30) && 10 * live <= 9 * warps;
+}
+
+cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char** why) {
+  AttnParams p = p_in;
+  static int sm_count[64] = {0};                          // per device, asked once
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+    if (sm_count[dev] == 0 &&
+        cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sm_count[dev] = 148;
+    sms = sm_count[dev];
+  }
+  // A packed batch runs on the one-tile kernels without the negligible-tile tests: its sequences
+  // differ in length, and the smaller unit of work evens them out.
+  const bool varlen = p.cu_q != nullptr;
+  const int forced = g_force_tiles_per_cta.load(std::memory_order_relaxed);
+  bool two = choose_tiles_per_cta((p.Nq + TILE - 1) / TILE, p.B * p.Hq, p.causal != 0, sms) == 2;
+  // A loop over few key tiles is mostly start and end of a CTA, which only a second CTA on the SM
+  // hides: 40 heads x 16 384 queries x 512 keys 235 us with one tile, 265 with two; 48 x 288 x 288
+  // 12.7 / 14.4; 2 x 24 x 1 000 x 1 000 39.4 / 45.5; but 48 x 2 048 x 2 048 (16 key tiles) 121 / 118.
+  if (p.N_pad <= 8 * TILE) two = false;
+  if (forced != 0) two = (forced == 2);
+  if (varlen) two = false;
+  // Which of the two sets of kernels: with the negligible-tile tests (the default) or without.
+  // The threshold hook at 0 and the caller's `no_fast_path` both select the plain set.
+  const float skip = g_skip_log2.load(std::memory_order_relaxed);
+  const bool fast = !p.no_fast_path && skip > 0.f && !varlen;
+  const int n_split = (p.part && !p.causal && !varlen && forced == 0)
+                          ? key_splits(p.B, p.Hq, p.H, p.Nq, p.N, std::min(sms, SPLIT_SIZING_SMS)) : 1;
+  const bool ragged = n_split > 1 || (!p.causal && !varlen && !fast && !two && mostly_empty_tiles(p));
+  const int fold = ragged ? (int)(p.Hq / p.H) : 1;
+  if (ragged) { p.Nq = p_in.Nq * fold; p.Hq = p.H; }
   const uint64_t bh = (uint64_t)(p.B * p.H), N_pad = (uint64_t)p.N_pad;
   const uint64_t bhq = (uint64_t)(p.B * p.Hq), Nq = (uint64_t)p.Nq;
   CUtensorMap mq, mk, mv;
@@ -1041,34 +1218,38 @@ cudaError_t launch_attention(const AttnParams& p, cudaStream_t st, const char** 
   ka.Nq = p.Nq; ka.Hq = p.Hq; ka.group = p.Hq / p.H; ka.lse = p.lse; ka.qm = p.qm; ka.D = (int)p.D; ka.vmean = p.vmean;
   ka.o_sb = p.o_strides[0]; ka.o_sh = p.o_strides[1]; ka.o_sr = p.o_strides[2];
   ka.sm_scale = p.sm_scale; ka.status = p.status;
+  ka.rows_per_head = (int)p_in.Nq; ka.heads_per_unit = fold;
+  ka.splits = 1; ka.split_tiles = 0; ka.part_o = nullptr; ka.part_ml = nullptr; ka.part_max = nullptr;
   const unsigned q_tiles = (unsigned)((p.Nq + TILE - 1) / TILE);
-  static int sm_count[64] = {0};                          // per device, asked once
-  int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
-    if (sm_count[dev] == 0 &&
-        cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sm_count[dev] = 148;
-    sms = sm_count[dev];
-  }
-  bool two = choose_tiles_per_cta((int64_t)q_tiles, (int64_t)bhq, p.causal != 0, sms) == 2;
-  const int forced = g_force_tiles_per_cta.load(std::memory_order_relaxed);
-  if (forced != 0) two = (forced == 2);
-  // A packed batch runs on the one-tile kernels without the negligible-tile tests: its sequences
-  // differ in length, and the smaller unit of work evens them out.
-  const bool varlen = p.cu_q != nullptr;
   ka.cu_q = p.cu_q; ka.cu_k = p.cu_k; ka.Tq = p.Tq; ka.Tk = p.Tk;
-  if (varlen) two = false;
   dim3 grid(two ? (q_tiles + 1) / 2 : q_tiles, (unsigned)bhq);
-  // Which of the two sets of kernels: with the negligible-tile tests (the default) or without.
-  // The threshold hook at 0 and the caller's `no_fast_path` both select the plain set.
-  const float skip = g_skip_log2.load(std::memory_order_relaxed);
-  const bool fast = !p.no_fast_path && skip > 0.f && !varlen;
   ka.skip_log2 = skip;
   ka.skipped = fast ? p.skipped : nullptr;
+  if (n_split > 1) {
+    const int key_tiles = (int)(p.N_pad / TILE);
+    const long long rows = (long long)(bhq * Nq);
+    ka.split_tiles = (key_tiles + n_split - 1) / n_split;
+    ka.splits = (key_tiles + ka.split_tiles - 1) / ka.split_tiles;     // every share has a key tile
+    ka.part_o = reinterpret_cast<float*>(p.part);
+    ka.part_ml = reinterpret_cast<float2*>(ka.part_o + (size_t)ka.splits * rows * HD);
+    ka.part_max = reinterpret_cast<float*>(ka.part_ml + (size_t)ka.splits * rows);
+    const dim3 sgrid(q_tiles * (unsigned)ka.splits, (unsigned)bhq);
+    cudaError_t es = p.qk_mode == 0 ? launch_inst<true, false, __half, 1, false, false, SPLIT_MAX>(mq, mk, mv, ka, sgrid, st)
+                                    : launch_inst<false, false, __half, 1, false, false, SPLIT_MAX>(mq, mk, mv, ka, sgrid, st);
+    if (es == cudaSuccess)
+      es = p.qk_mode == 0 ? launch_inst<true, false, __half, 1, false, false, SPLIT_SUM>(mq, mk, mv, ka, sgrid, st)
+                          : launch_inst<false, false, __half, 1, false, false, SPLIT_SUM>(mq, mk, mv, ka, sgrid, st);
+    if (es == cudaSuccess)
+      es = launch_after_predecessor(p.out_dtype == 0 ? combine_splits_kernel<__half> : combine_splits_kernel<__nv_bfloat16>,
+                                    dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, st, ka, rows);
+    if (es != cudaSuccess && why) *why = "attention kernel launch failed";
+    return es;
+  }
   const int key = (p.qk_mode == 0 ? 4 : 0) | (p.causal ? 2 : 0) | (p.out_dtype == 0 ? 1 : 0);
   cudaError_t e;
 #define SAGE_LAUNCH(I8, C, T)                                                                          \
   e = varlen ? launch_inst<I8, C, T, 1, false, true>(mq, mk, mv, ka, grid, st) :                       \
+      ragged ? launch_inst<I8, false, T, 1, false, false, RAGGED>(mq, mk, mv, ka, grid, st) :          \
       two ? (fast ? launch_inst<I8, C, T, 2, true>(mq, mk, mv, ka, grid, st)                           \
                   : launch_inst<I8, C, T, 2, false>(mq, mk, mv, ka, grid, st))                         \
           : (fast ? launch_inst<I8, C, T, 1, true>(mq, mk, mv, ka, grid, st)                           \

@@ -97,7 +97,7 @@ struct Packed {
 constexpr Packed kNotPacked = {nullptr, nullptr, 0, 0};
 
 struct Layout {
-  size_t q8, sq, k8, sk, v8t, sv, svp, s_fold, mean, ctrl, status, qm, vmean, total;
+  size_t q8, sq, k8, sk, v8t, sv, svp, s_fold, mean, ctrl, status, qm, vmean, base_total, part, total;
 };
 
 Layout carve(const Dims& d) {
@@ -121,6 +121,8 @@ Layout carve(const Dims& d) {
   L.status = L.ctrl + 4 * (sage::CtrlHeader::status_word((int64_t)bhk) + 1);
   L.qm = take(bhq * nq * 4);
   L.vmean = take(bhk * sage::HD * 4);
+  L.base_total = off;               // what a call needs; with the rest it may split its keys over CTAs
+  L.part = take(sage::split_scratch_bytes(d.B, d.Hq, d.Hkv, d.Nq, d.Nk));
   L.total = off;
   return L;
 }
@@ -163,7 +165,7 @@ int attn_impl(const void* q8, const float* sq, const void* k8, const float* sk,
               const void* v8t, const float* svp, const float* s_fold, void* out, float* lse, const float* qm,
               const float* vmean, const Dims& d, int64_t Nk_pad, const int64_t o_strides[3],
               int causal, float sm_scale, int out_dtype, int qk_mode, int32_t* status, void* stream,
-              const char* who, unsigned* skipped = nullptr, const Packed& pk = kNotPacked) {
+              const char* who, unsigned* skipped = nullptr, const Packed& pk = kNotPacked, void* part = nullptr) {
   g_err[0] = 0;
   int rc = check_dims(d);
   if (rc) return rc;
@@ -192,6 +194,7 @@ int attn_impl(const void* q8, const float* sq, const void* k8, const float* sk,
   p.status = status;
   p.no_fast_path = no_fast_path; p.skipped = skipped;
   p.cu_q = pk.cu_q; p.cu_k = pk.cu_k; p.Tq = pk.Tq; p.Tk = pk.Tk;
+  p.part = part;
   const char* why = nullptr;
   cudaError_t e = sage::launch_attention(p, reinterpret_cast<cudaStream_t>(stream), &why);
   if (e != cudaSuccess) return fail(SAGE_E_CUDA, "%s: %s (%s)", who, why ? why : "", cudaGetErrorString(e));
@@ -210,8 +213,8 @@ int attention_impl(const void* q, const void* k, const void* v, void* out, float
   if (!workspace) return fail(SAGE_E_ARG, "%s: workspace is null", who);
   if (reinterpret_cast<uintptr_t>(workspace) & 255u) return fail(SAGE_E_ARG, "%s: workspace must be 256-byte aligned", who);
   const Layout L = carve(d);
-  if (workspace_bytes < L.total)
-    return fail(SAGE_E_WORKSPACE, "%s: workspace has %zu bytes, needs %zu", who, workspace_bytes, L.total);
+  if (workspace_bytes < L.base_total)
+    return fail(SAGE_E_WORKSPACE, "%s: workspace has %zu bytes, needs %zu", who, workspace_bytes, L.base_total);
   // what the attention step would refuse is refused before the prologue is launched
   if (!out) return fail(SAGE_E_ARG, "%s: null pointer argument", who);
   if (causal && d.Nq != d.Nk) return fail(SAGE_E_ARG, "%s: a causal call needs as many queries as keys", who);
@@ -237,7 +240,8 @@ int attention_impl(const void* q, const void* k, const void* v, void* out, float
                    reinterpret_cast<float*>(w + L.sk), w + L.v8t, reinterpret_cast<float*>(w + L.svp),
                    reinterpret_cast<float*>(w + L.s_fold), out, lse, qm, vmean, d, Nk_pad, o_strides,
                    causal, sm_scale, dtype, qk_mode | flags, status, stream, who,
-                   reinterpret_cast<unsigned*>(status) + 3, pk);
+                   reinterpret_cast<unsigned*>(status) + 3, pk,
+                   (L.total > L.base_total && workspace_bytes >= L.total) ? w + L.part : nullptr);
 }
 
 }  // namespace

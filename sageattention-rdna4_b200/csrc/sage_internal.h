@@ -50,6 +50,7 @@ struct AttnParams {
   unsigned* skipped;                                   // optional: (warp, key tile) pairs the fast path skipped
   const int32_t *cu_q, *cu_k;                          // packed variable-length batch (see PrologueParams); null otherwise
   int64_t Tq, Tk;                                      // with cu_q / cu_k: tokens in the packed tensors
+  void* part;                                          // optional: split_scratch_bytes() of scratch; without it the keys of a call are not split
 };
 
 cudaError_t launch_prologue(const PrologueParams& p, cudaStream_t st);
@@ -57,6 +58,12 @@ size_t prologue_ctrl_bytes(int64_t B, int64_t H, int64_t N);
 
 // Returns cudaSuccess or an error; `why` (if non-null) receives a static description on failure.
 cudaError_t launch_attention(const AttnParams& p, cudaStream_t st, const char** why);
+
+// Scratch for the partial results of a call whose keys are split over CTAs (0: never split); sized
+// without a device at hand, for the largest SM count an sm_100 part has.
+constexpr int SPLIT_SIZING_SMS = 160;
+int key_splits(int64_t B, int64_t Hq, int64_t H, int64_t Nq, int64_t Nk, int sms);
+size_t split_scratch_bytes(int64_t B, int64_t Hq, int64_t H, int64_t Nq, int64_t Nk);
 
 // Test hook: force the attention kernel's shape (1 or 2 query tiles per CTA; 0 = automatic).
 void set_tiles_per_cta(int n);
