@@ -304,6 +304,8 @@ struct AttnKArgs {
   float* part_max;    // SPLIT kernels: (splits, units x rows) largest score of the share, in the u domain
   const int *cu_q, *cu_k;   // VARLEN kernels: cumulative token counts of the packed batch (B + 1 entries each)
   long long Tq, Tk;         // VARLEN kernels: tokens in the packed q / out and k / v tensors
+  const int* plan;          // VARLEN kernels, optional: the batch's work list (see plan_packed_kernel)
+  int n_seq;
 };
 
 template <typename OutT> __device__ __forceinline__ uint32_t pack2(float a, float b);
@@ -353,11 +355,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // first query tile of this CTA (causal: longest first); softmax group g owns tile q_tile0 + g
-  const int q_tile0 = NQ * (CAUSAL ? (int)(gridDim.x - 1 - blockIdx.x)
+  int q_tile0 = NQ * (CAUSAL ? (int)(gridDim.x - 1 - blockIdx.x)
                                    : SPLIT ? (int)blockIdx.x / a.splits : (int)blockIdx.x);
   const int share = SPLIT ? (int)blockIdx.x % a.splits : 0;
   const int k_tile0 = SPLIT ? share * a.split_tiles : 0;     // first key tile of this CTA
-  const int bh = blockIdx.y;                          // (batch, query head)
+  int bh = blockIdx.y;                                // (batch, query head)
+  if (VARLEN && a.plan != nullptr) {
+    // the blockIdx.x-th query tile that exists: sequences in the order of the work list (longest
+    // first), head by head; 32 of the list's prefix sums at a time
+    const int x = (int)blockIdx.x, hq = (int)a.Hq;
+    const int* pre = a.plan + a.n_seq + 1;
+    if (x >= pre[a.n_seq] * hq) return;
+    int s = 0;
+    for (;; s += 32) {
+      const unsigned below = __ballot_sync(0xffffffffu, s + lane < a.n_seq && pre[min(s + lane, a.n_seq - 1) + 1] * hq <= x);
+      if (below != 0xffffffffu) { s += __popc(below); break; }
+    }
+    const int rem = x - pre[s] * hq, per = pre[s + 1] - pre[s];
+    bh = a.plan[s] * hq + rem / per;
+    q_tile0 = CAUSAL ? per - 1 - rem % per : rem % per;
+  }
   const int bh_kv = (int)((bh / a.Hq) * a.H + (bh % a.Hq) / a.group);   // its (batch, K/V head)
   // Key tiles query tile g visits: all of them, or when causal those up to its diagonal (a causal
   // call has as many key tiles as query tiles; the second tile of the last CTA may not exist, it
@@ -1222,7 +1239,12 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
   ka.splits = 1; ka.split_tiles = 0; ka.part_o = nullptr; ka.part_ml = nullptr; ka.part_max = nullptr;
   const unsigned q_tiles = (unsigned)((p.Nq + TILE - 1) / TILE);
   ka.cu_q = p.cu_q; ka.cu_k = p.cu_k; ka.Tq = p.Tq; ka.Tk = p.Tk;
+  ka.plan = p.plan; ka.n_seq = (int)p.B;
   dim3 grid(two ? (q_tiles + 1) / 2 : q_tiles, (unsigned)bhq);
+  // With a work list the grid covers the tiles that sequences of Tq tokens in all can have, in
+  // slots of the longest length at most.
+  if (varlen && p.plan)
+    grid = dim3((unsigned)(std::min<int64_t>(p.Tq / TILE + p.B, p.B * (int64_t)q_tiles) * p.Hq));
   ka.skip_log2 = skip;
   ka.skipped = fast ? p.skipped : nullptr;
   if (n_split > 1) {

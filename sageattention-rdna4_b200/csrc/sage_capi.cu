@@ -93,8 +93,19 @@ int check_dims(const Dims& d) {
 struct Packed {
   const int32_t *cu_q, *cu_k;
   int64_t Tq, Tk;
+  void* scratch;                 // optional: room for the batch's work list and the partial sums of its means
+  size_t scratch_bytes;
 };
-constexpr Packed kNotPacked = {nullptr, nullptr, 0, 0};
+constexpr Packed kNotPacked = {nullptr, nullptr, 0, 0, nullptr, 0};
+
+// The work list of a packed batch sits at the start of its scratch, if that is large enough.  The
+// quantiser counts its items in 31 bits.
+int* packed_plan(const Dims& d, const Packed& pk) {
+  const size_t need = sage::plan_bytes(d.B);
+  const int64_t items = d.B * (d.Hq * ((d.Nq + sage::TILE - 1) / sage::TILE) + 2 * d.Hkv * ((d.Nk + sage::TILE - 1) / sage::TILE));
+  return (need && pk.scratch && align256(need) <= pk.scratch_bytes && items < ((int64_t)1 << 30))
+             ? reinterpret_cast<int*>(pk.scratch) : nullptr;
+}
 
 struct Layout {
   size_t q8, sq, k8, sk, v8t, sv, svp, s_fold, mean, ctrl, status, qm, vmean, base_total, part, total;
@@ -156,6 +167,10 @@ int prologue_impl(const void* q, const void* k, const void* v,
   for (int i = 0; i < 3; ++i) { p.q_strides[i] = q_strides[i]; p.k_strides[i] = k_strides[i]; p.v_strides[i] = v_strides[i]; }
   p.dtype = dtype; p.qk_mode = qk_mode; p.smooth_k = smooth_k;
   p.cu_q = pk.cu_q; p.cu_k = pk.cu_k; p.Tq = pk.Tq; p.Tk = pk.Tk;
+  p.plan = packed_plan(d, pk);
+  const size_t plan_room = p.plan ? align256(sage::plan_bytes(d.B)) : 0;
+  p.partial = pk.scratch ? reinterpret_cast<char*>(pk.scratch) + plan_room : nullptr;
+  p.partial_bytes = pk.scratch_bytes > plan_room ? pk.scratch_bytes - plan_room : 0;
   cudaError_t e = sage::launch_prologue(p, reinterpret_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(SAGE_E_CUDA, "%s: %s", who, cudaGetErrorString(e));
   return SAGE_OK;
@@ -194,6 +209,7 @@ int attn_impl(const void* q8, const float* sq, const void* k8, const float* sk,
   p.status = status;
   p.no_fast_path = no_fast_path; p.skipped = skipped;
   p.cu_q = pk.cu_q; p.cu_k = pk.cu_k; p.Tq = pk.Tq; p.Tk = pk.Tk;
+  p.plan = packed_plan(d, pk);
   p.part = part;
   const char* why = nullptr;
   cudaError_t e = sage::launch_attention(p, reinterpret_cast<cudaStream_t>(stream), &why);
@@ -206,7 +222,7 @@ int attention_impl(const void* q, const void* k, const void* v, void* out, float
                    const int64_t q_strides[3], const int64_t k_strides[3],
                    const int64_t v_strides[3], const int64_t o_strides[3],
                    int dtype, int qk_mode, int causal, int smooth_k, int smooth_v, float sm_scale, void* stream,
-                   const char* who, const Packed& pk = kNotPacked) {
+                   const char* who, Packed pk = kNotPacked) {
   g_err[0] = 0;
   int rc = check_dims(d);
   if (rc) return rc;
@@ -229,6 +245,7 @@ int attention_impl(const void* q, const void* k, const void* v, void* out, float
   const int64_t Nk_pad = sage_pad_len(d.Nk);
   int32_t* status = reinterpret_cast<int32_t*>(w + L.status);     // zeroed by the prologue's clearing kernel
   float* qm = (lse && smooth_k) ? reinterpret_cast<float*>(w + L.qm) : nullptr;
+  if (pk.cu_q) { pk.scratch = w + L.qm; pk.scratch_bytes = L.vmean - L.qm; }   // a packed batch has no LSE
   float* vmean = smooth_v ? reinterpret_cast<float*>(w + L.vmean) : nullptr;
   rc = prologue_impl(q, k, v, w + L.q8, reinterpret_cast<float*>(w + L.sq), w + L.k8,
                      reinterpret_cast<float*>(w + L.sk), w + L.v8t, reinterpret_cast<float*>(w + L.sv),
@@ -425,7 +442,7 @@ int sage_attention_varlen(const void* q, const void* k, const void* v, void* out
   const int64_t qs[3] = {q_strides[0], q_strides[1], q_strides[0]}, ks[3] = {k_strides[0], k_strides[1], k_strides[0]};
   const int64_t vs[3] = {v_strides[0], v_strides[1], v_strides[0]}, os[3] = {o_strides[0], o_strides[1], o_strides[0]};
   const Dims d = {n_seq, Hq, Hkv, max_q, max_k, head_dim};
-  const Packed pk = {cu_seqlens_q, cu_seqlens_k, total_q, total_k};
+  const Packed pk = {cu_seqlens_q, cu_seqlens_k, total_q, total_k, nullptr, 0};
   return attention_impl(q, k, v, out, nullptr, workspace, workspace_bytes, d, qs, ks, vs, os, dtype, qk_mode,
                         causal, smooth_k, 0, sm_scale, stream, "sage_attention_varlen", pk);
 }

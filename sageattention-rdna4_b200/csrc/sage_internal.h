@@ -28,7 +28,14 @@ struct PrologueParams {
   // outputs, Tq / Tk the token counts of the packed tensors.
   const int32_t *cu_q, *cu_k;
   int64_t Tq, Tk;
+  int* plan;                 // packed batch, optional: plan_bytes(B) of scratch for the work list, which the attention kernel reads too
+  void* partial;             // packed batch, optional: more room for the partial sums of the mean kernel
+  size_t partial_bytes;
 };
+
+// Work list of a packed batch (see plan_packed_kernel); batches of more sequences go without.
+constexpr int PLAN_MAX_SEQS = 512;
+inline size_t plan_bytes(int64_t B) { return B <= PLAN_MAX_SEQS ? (size_t)4 * (size_t)(B + 1) * sizeof(int) : 0; }
 
 struct AttnParams {
   const void *q8, *k8, *v8t;
@@ -50,6 +57,7 @@ struct AttnParams {
   unsigned* skipped;                                   // optional: (warp, key tile) pairs the fast path skipped
   const int32_t *cu_q, *cu_k;                          // packed variable-length batch (see PrologueParams); null otherwise
   int64_t Tq, Tk;                                      // with cu_q / cu_k: tokens in the packed tensors
+  const int* plan;                                     // packed batch, optional: the prologue's work list
   void* part;                                          // optional: split_scratch_bytes() of scratch; without it the keys of a call are not split
 };
 

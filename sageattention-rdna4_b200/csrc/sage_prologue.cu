@@ -30,6 +30,8 @@
 
 namespace sage {
 
+constexpr int FOLD_KEYS = 4096;     // keys per fold item of the quantiser
+
 // ------------------------------------------------------------------------------------------------
 // Kernel 0: clears the control words (arrival counters, running maxima, status words, work and
 // skip counters) of a call.  A kernel rather than a memset so that it and the mean kernel behind it
@@ -40,6 +42,55 @@ __global__ void __launch_bounds__(256) clear_ctrl_kernel(unsigned* __restrict__ 
   wait_for_predecessor();            // an earlier call may still be using these words
   allow_successor();
   for (int i = threadIdx.x; i < n; i += 256) words[i] = 0u;
+}
+
+// The same for a packed batch, and the batch's work list: the sequences ordered by their work,
+// longest first, and in that order the prefix sums of their query tiles, key tiles and fold items
+// (plan: four arrays of B + 1 words).  The kernels behind it then draw only tiles that exist; in
+// slots of the longest length, 59 % of the quantiser's items and of the attention grid were empty
+// in a batch of eleven sequences of 512 .. 8 192 tokens.  One block: a few microseconds for up to
+// PLAN_MAX_SEQS sequences.
+__global__ void __launch_bounds__(PLAN_MAX_SEQS)
+plan_packed_kernel(unsigned* __restrict__ words, int n, int* __restrict__ plan, int B,
+                   const int* __restrict__ cu_q, const int* __restrict__ cu_k, long long Tq, long long Tk,
+                   long long Nq, long long Nk) {
+  __shared__ long long s_work[PLAN_MAX_SEQS];
+  __shared__ int s_pre[3][PLAN_MAX_SEQS];
+  wait_for_predecessor();
+  allow_successor();
+  const int tid = threadIdx.x;
+  for (int i = tid; i < n; i += PLAN_MAX_SEQS) words[i] = 0u;
+  // a sequence's live length, clamped to the packed tensor and to its slot as in the other kernels
+  auto tiles = [&](const int* cu, long long T, long long cap) {
+    const long long s0 = min(max((long long)cu[tid], 0LL), T), s1 = min((long long)cu[tid + 1], T);
+    return (int)((min(max(s1 - s0, 0LL), cap) + TILE - 1) / TILE);
+  };
+  int tq = 0, tk = 0;
+  if (tid < B) { tq = tiles(cu_q, Tq, Nq); tk = tiles(cu_k, Tk, Nk); }
+  const long long work = (long long)tq * tk;
+  s_work[tid] = work;
+  s_pre[0][tid] = 0; s_pre[1][tid] = 0; s_pre[2][tid] = 0;
+  __syncthreads();
+  if (tid < B) {
+    int rank = 0;
+    for (int i = 0; i < B; ++i) rank += (s_work[i] > work || (s_work[i] == work && i < tid)) ? 1 : 0;
+    plan[rank] = tid;
+    s_pre[0][rank] = tq; s_pre[1][rank] = tk; s_pre[2][rank] = (tk * TILE + FOLD_KEYS - 1) / FOLD_KEYS;
+  }
+  __syncthreads();
+  for (int off = 1; off < PLAN_MAX_SEQS; off <<= 1) {        // inclusive scan of the three arrays
+    int v[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[a] = (tid >= off) ? s_pre[a][tid - off] : 0;
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) s_pre[a][tid] += v[a];
+    __syncthreads();
+  }
+  if (tid < 3) plan[(tid + 1) * (B + 1)] = 0;
+  if (tid < B)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) plan[(a + 1) * (B + 1) + tid + 1] = s_pre[a][tid];
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -66,6 +117,8 @@ kmean_kernel(const T* __restrict__ K, float* __restrict__ mean, double* __restri
     N = min(max(s1 - s0, 0LL), N);
     base = K + s0 * sr + h * sh + 8 * c;
   }
+  const int n_arrive = VARLEN ? max((int)((N + chunk - 1) / chunk), 1) : nsplit;   // CTAs of this head with tokens
+  if (VARLEN && split >= n_arrive) return;
   const long long n0 = (long long)split * chunk;
   const long long n1 = min(N, n0 + chunk);
 
@@ -92,12 +145,12 @@ kmean_kernel(const T* __restrict__ K, float* __restrict__ mean, double* __restri
   }
   __threadfence();
   __syncthreads();
-  if (tid == 0) s_last = (atomicAdd(&arrivals[bh], 1u) == (unsigned)(nsplit - 1));
+  if (tid == 0) s_last = (atomicAdd(&arrivals[bh], 1u) == (unsigned)(n_arrive - 1));
   __syncthreads();
   if (s_last && tid < HD) {
     __threadfence();
     double tot = 0.0;
-    for (int sp = 0; sp < nsplit; ++sp) tot += __ldcg(&partial[((size_t)bh * nsplit + sp) * HD + tid]);
+    for (int sp = 0; sp < n_arrive; ++sp) tot += __ldcg(&partial[((size_t)bh * nsplit + sp) * HD + tid]);
     mean[(size_t)bh * HD + tid] = (!VARLEN || N > 0) ? (float)(tot / (double)N) : 0.f;
   }
 }
@@ -128,6 +181,8 @@ struct QuantArgs {
   unsigned long long* next_item;  // global work counter (zeroed with the control block)
   const int *cu_q, *cu_k;         // VARLEN kernels: cumulative token counts of the packed batch (B + 1 entries each)
   long long Tq, Tk;               // VARLEN kernels: tokens in the packed q and k/v tensors
+  const int* plan;                // VARLEN kernels, optional: the work list of plan_packed_kernel
+  int n_seq;
 };
 
 // rn(x / s) given rc = rn(1/s)
@@ -148,7 +203,6 @@ __device__ __forceinline__ float div_by_scale(float x, float s, float rc) {
 // ------------------------------------------------------------------------------------------------
 constexpr int QT_STAGES = 2;        // shared-memory ring: one tile being quantised, one in flight
 constexpr int QT_MINBLOCKS = 3;     // CTAs per SM (3 x 64 KB of shared memory, 80 registers per thread)
-constexpr int FOLD_KEYS = 4096;     // keys per fold item
 constexpr uint32_t QT_STAGE_BYTES = TILE * HD * 2;
 constexpr uint32_t QT_SMEM_BYTES = QT_STAGES * QT_STAGE_BYTES + 128 /* alignment slack */ + 64 /* barriers */;
 constexpr long long QT_WAIT_CYCLES = 4000000000LL;
@@ -192,6 +246,7 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                      const __grid_constant__ CUtensorMap tm_v, const QuantArgs a) {
   extern __shared__ uint8_t qt_smem[];
   __shared__ long long s_item[QT_STAGES];
+  __shared__ int s_plan[VARLEN ? 4 * (PLAN_MAX_SEQS + 1) : 1];
   wait_for_predecessor();            // the means and the cleared control block
   allow_successor();                 // persistent grid: every CTA is resident
   constexpr float QMAX = INT8 ? I8_MAX : F8_MAX;
@@ -207,11 +262,37 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const long long items_k = a.BHkv * tiles_k, items_q = a.BHq * tiles_q;
   const long long fold_per_head = (a.N_pad + FOLD_KEYS - 1) / FOLD_KEYS;
   const long long items_f = a.BHkv * fold_per_head;
-  const long long total = 2 * items_k + items_q + items_f;
+  const bool planned = VARLEN && a.plan != nullptr;
+  const int P1 = VARLEN ? a.n_seq + 1 : 0;
+  if (planned) {
+    for (int i = tid; i < 4 * P1; i += 256) s_plan[i] = a.plan[i];
+    __syncthreads();
+  }
+  const long long live_k = planned ? s_plan[3 * P1 - 1] * a.H : items_k, live_q = planned ? s_plan[2 * P1 - 1] * a.Hq : items_q;
+  const long long total = 2 * live_k + live_q + (planned ? s_plan[4 * P1 - 1] * a.H : items_f);
 
   // item -> (tensor, head, tile): K first with the last heads first (their rows are still in L2
   // after the mean pass), then V (so that the per-head folds overlap the Q items), then Q
   auto decode = [&](long long it, int& which, long long& bh, long long& tile) {
+    if (planned) {                     // sequence by sequence in the plan's order, head by head
+      int arr = 2;
+      int j;
+      if (it < live_k) { which = 1; j = (int)it; }
+      else if (it < 2 * live_k) { which = 2; j = (int)(it - live_k); }
+      else if (it < 2 * live_k + live_q) { which = 0; j = (int)(it - 2 * live_k); arr = 1; }
+      else { which = 3; j = (int)(it - 2 * live_k - live_q); arr = 3; }
+      const int heads = (int)((which == 0) ? a.Hq : a.H);
+      const int* pre = s_plan + arr * P1;
+      int lo = 0, hi = a.n_seq;        // pre[lo] * heads <= j < pre[hi] * heads
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if ((long long)pre[mid] * heads <= j) lo = mid; else hi = mid;
+      }
+      const int rem = j - pre[lo] * heads, per = pre[lo + 1] - pre[lo];
+      bh = (long long)s_plan[lo] * heads + rem / per;
+      tile = rem % per;
+      return;
+    }
     if (it < items_k) { which = 1; bh = a.BHkv - 1 - it / tiles_k; tile = it % tiles_k; }
     else if (it < 2 * items_k) { const long long j = it - items_k; which = 2; bh = a.BHkv - 1 - j / tiles_k; tile = j % tiles_k; }
     else if (it < 2 * items_k + items_q) { const long long j = it - 2 * items_k; which = 0; bh = a.BHq - 1 - j / tiles_q; tile = j % tiles_q; }
@@ -597,9 +678,21 @@ static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
     e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
   }
-  e = launch_after_predecessor(clear_ctrl_kernel, dim3(1), dim3(256), 0, st, words, (int)CtrlHeader::words(bh));
+  if (p.plan)
+    e = launch_after_predecessor(plan_packed_kernel, dim3(1), dim3(PLAN_MAX_SEQS), 0, st, words, (int)CtrlHeader::words(bh),
+                                 p.plan, (int)p.B, p.cu_q, p.cu_k, (long long)p.Tq, (long long)p.Tk, (long long)p.Nq,
+                                 (long long)p.N);
+  else
+    e = launch_after_predecessor(clear_ctrl_kernel, dim3(1), dim3(256), 0, st, words, (int)CtrlHeader::words(bh));
   if (e != cudaSuccess) return e;
-  const int nsplit = std::min(kmean_splits(bh, p.N, sm_count[dev]), kmean_splits_max(bh, p.N));
+  int nsplit = std::min(kmean_splits(bh, p.N, sm_count[dev]), kmean_splits_max(bh, p.N));
+  // A packed batch: chunks of 1 024 tokens whatever the number of heads, since its longest sequence
+  // would otherwise keep single CTAs busy long after the others (36 k tokens x 48 heads in eleven
+  // sequences of up to 8 192: 262 us with one CTA per sequence and head).  CTAs past a sequence's end leave.
+  if (p.partial && p.cu_k) {
+    const int64_t want = std::min<int64_t>((p.N + 1023) / 1024, (int64_t)(p.partial_bytes / ((size_t)bh * HD * sizeof(double))));
+    if (want > nsplit) { nsplit = (int)std::min<int64_t>(want, 65535); partial = reinterpret_cast<double*>(p.partial); }
+  }
   if (p.smooth_k) {
     long long chunk = (p.N + nsplit - 1) / nsplit;
     chunk = (chunk + 15) / 16 * 16;
@@ -629,6 +722,7 @@ static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
   a.Nq = p.Nq; a.Hq = p.Hq; a.group = p.Hq / p.H; a.BHq = p.B * p.Hq; a.BHkv = bh; a.qm = p.qm;
   a.sub_mean = p.smooth_k ? 1 : 0;
   a.cu_q = p.cu_q; a.cu_k = p.cu_k; a.Tq = p.Tq; a.Tk = p.Tk;
+  a.plan = p.plan; a.n_seq = (int)p.B;
   const bool varlen = p.cu_q != nullptr;
   const int64_t tq = (p.Nq + TILE - 1) / TILE, tk = p.N_pad / TILE;
   a.status = reinterpret_cast<int32_t*>(words + CtrlHeader::status_word(bh));
