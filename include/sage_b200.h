@@ -242,6 +242,36 @@ int sage_attention_ex(const void* q, const void* k, const void* v, void* out, fl
 int sage_workspace_layout_ex(int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk,
                              size_t offsets[13]);
 
+/* sage_attention_ex, sage_attention_varlen and sage_attn_fwd_ex with one more argument.
+ * `status_host` (may be null) is a 4-byte word of pinned host memory that the device can write
+ * (cudaHostAlloc / cudaHostRegister).  When a bounded wait of the call has run out, the attention
+ * kernel writes the call's status word there; a call that succeeds writes nothing, so that a host
+ * learns of a failure without a copy behind every call.  The word must stay allocated until the
+ * call has finished; a captured call keeps using it in every replay. */
+int sage_attention_reported(const void* q, const void* k, const void* v, void* out, float* lse,
+                            void* workspace, size_t workspace_bytes,
+                            int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int64_t head_dim,
+                            const int64_t q_strides[3], const int64_t k_strides[3],
+                            const int64_t v_strides[3], const int64_t o_strides[3],
+                            int dtype, int qk_mode, int causal, int smooth_k, int smooth_v, float sm_scale,
+                            int32_t* status_host, void* stream);
+int sage_attention_varlen_reported(const void* q, const void* k, const void* v, void* out,
+                                   const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
+                                   void* workspace, size_t workspace_bytes,
+                                   int64_t n_seq, int64_t Hq, int64_t Hkv,
+                                   int64_t total_q, int64_t total_k, int64_t max_q, int64_t max_k,
+                                   int64_t head_dim,
+                                   const int64_t q_strides[2], const int64_t k_strides[2],
+                                   const int64_t v_strides[2], const int64_t o_strides[2],
+                                   int dtype, int qk_mode, int causal, int smooth_k, float sm_scale,
+                                   int32_t* status_host, void* stream);
+int sage_attn_fwd_reported(const void* q8, const float* sq, const void* k8, const float* sk,
+                           const void* v8t, const float* svp, const float* s_fold, void* out,
+                           float* lse, const float* qm, const float* vmean,
+                           int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int64_t Nk_pad,
+                           int64_t head_dim, const int64_t o_strides[3], int causal, float sm_scale, int out_dtype,
+                           int qk_mode, int32_t* status, int32_t* status_host, void* stream);
+
 /* ---- A packed variable-length batch in one call: replaces `sageattn_varlen`
  * (sageattention/core.py:1444-1558), whose per-block quantisers take `cu_seqlens` and whose kernel
  * is launched once for the whole batch.  The cumulative lengths stay on the device: nothing is read

@@ -296,6 +296,7 @@ struct AttnKArgs {
   float skip_log2;    // FAST kernels: key tiles whose scores all lie this far (exponent domain) below the running maxima are not exponentiated
   unsigned* skipped;  // FAST kernels, optional: receives the number of (warp, key tile) pairs that were skipped
   int32_t* status;
+  int32_t* status_host;   // optional, pinned host memory: receives the status word of a call that failed
   int rows_per_head;  // query rows of one head: Nq, unless grouped heads are folded into one unit (see launch_attention)
   int heads_per_unit; // heads folded into one unit (1: none)
   int splits, split_tiles;  // SPLIT kernels: shares of the key range, key tiles in a share
@@ -1016,6 +1017,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (*cta_abort) {
+    // The host sees a failure through this one word; a call that succeeds writes nothing.  (Every
+    // thread writes it: an index kept to this point costs the kernels spilled registers.)
+    if (a.status_host != nullptr) {
+      *reinterpret_cast<volatile int32_t*>(a.status_host) = *reinterpret_cast<volatile int32_t*>(a.status);
+    }
     const long long t0 = clock64();
     while (clock64() - t0 < 400000) { }
     __syncthreads();
@@ -1214,7 +1220,8 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
   // Which of the two sets of kernels: with the negligible-tile tests (the default) or without.
   // The threshold hook at 0 and the caller's `no_fast_path` both select the plain set.
   const float skip = g_skip_log2.load(std::memory_order_relaxed);
-  const bool fast = !p.no_fast_path && skip > 0.f && !varlen;
+  // (Nor do loops over few key tiles take the tests: most of such a CTA's time is its start and end.)
+  const bool fast = !p.no_fast_path && skip > 0.f && !varlen && p.N_pad > 8 * TILE;
   const int n_split = (p.part && !p.causal && !varlen && forced == 0)
                           ? key_splits(p.B, p.Hq, p.H, p.Nq, p.N, std::min(sms, SPLIT_SIZING_SMS)) : 1;
   const bool ragged = n_split > 1 || (!p.causal && !varlen && !fast && !two && mostly_empty_tiles(p));
@@ -1234,7 +1241,7 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
   ka.N = p.N; ka.N_pad = p.N_pad; ka.H = p.H;
   ka.Nq = p.Nq; ka.Hq = p.Hq; ka.group = p.Hq / p.H; ka.lse = p.lse; ka.qm = p.qm; ka.D = (int)p.D; ka.vmean = p.vmean;
   ka.o_sb = p.o_strides[0]; ka.o_sh = p.o_strides[1]; ka.o_sr = p.o_strides[2];
-  ka.sm_scale = p.sm_scale; ka.status = p.status;
+  ka.sm_scale = p.sm_scale; ka.status = p.status; ka.status_host = p.status_host;
   ka.rows_per_head = (int)p_in.Nq; ka.heads_per_unit = fold;
   ka.splits = 1; ka.split_tiles = 0; ka.part_o = nullptr; ka.part_ml = nullptr; ka.part_max = nullptr;
   const unsigned q_tiles = (unsigned)((p.Nq + TILE - 1) / TILE);

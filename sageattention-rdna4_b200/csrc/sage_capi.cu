@@ -180,7 +180,8 @@ int attn_impl(const void* q8, const float* sq, const void* k8, const float* sk,
               const void* v8t, const float* svp, const float* s_fold, void* out, float* lse, const float* qm,
               const float* vmean, const Dims& d, int64_t Nk_pad, const int64_t o_strides[3],
               int causal, float sm_scale, int out_dtype, int qk_mode, int32_t* status, void* stream,
-              const char* who, unsigned* skipped = nullptr, const Packed& pk = kNotPacked, void* part = nullptr) {
+              const char* who, unsigned* skipped = nullptr, const Packed& pk = kNotPacked, void* part = nullptr,
+              int32_t* status_host = nullptr) {
   g_err[0] = 0;
   int rc = check_dims(d);
   if (rc) return rc;
@@ -210,7 +211,7 @@ int attn_impl(const void* q8, const float* sq, const void* k8, const float* sk,
   p.no_fast_path = no_fast_path; p.skipped = skipped;
   p.cu_q = pk.cu_q; p.cu_k = pk.cu_k; p.Tq = pk.Tq; p.Tk = pk.Tk;
   p.plan = packed_plan(d, pk);
-  p.part = part;
+  p.part = part; p.status_host = status_host;
   const char* why = nullptr;
   cudaError_t e = sage::launch_attention(p, reinterpret_cast<cudaStream_t>(stream), &why);
   if (e != cudaSuccess) return fail(SAGE_E_CUDA, "%s: %s (%s)", who, why ? why : "", cudaGetErrorString(e));
@@ -222,7 +223,7 @@ int attention_impl(const void* q, const void* k, const void* v, void* out, float
                    const int64_t q_strides[3], const int64_t k_strides[3],
                    const int64_t v_strides[3], const int64_t o_strides[3],
                    int dtype, int qk_mode, int causal, int smooth_k, int smooth_v, float sm_scale, void* stream,
-                   const char* who, Packed pk = kNotPacked) {
+                   const char* who, int32_t* status_host = nullptr, Packed pk = kNotPacked) {
   g_err[0] = 0;
   int rc = check_dims(d);
   if (rc) return rc;
@@ -238,6 +239,7 @@ int attention_impl(const void* q, const void* k, const void* v, void* out, float
   if (!aligned16(out)) return fail(SAGE_E_ARG, "%s: pointers must be 16-byte aligned", who);
   if (!(sm_scale > 0.f) || !(sm_scale <= 3.0e38f))
     return fail(SAGE_E_ARG, "%s: sm_scale must be finite and positive (got %g)", who, (double)sm_scale);
+  if (reinterpret_cast<uintptr_t>(status_host) & 3u) return fail(SAGE_E_ARG, "%s: status_host must be 4-byte aligned", who);
   const int flags = (qk_mode >= 0) ? (qk_mode & SAGE_QK_NO_FAST_PATH) : (((-qk_mode) & SAGE_QK_NO_FAST_PATH));
   if (qk_mode < 0) qk_mode = (dtype == SAGE_BF16) ? SAGE_QK_E4M3 : SAGE_QK_INT8;
   else qk_mode &= ~SAGE_QK_NO_FAST_PATH;
@@ -258,7 +260,7 @@ int attention_impl(const void* q, const void* k, const void* v, void* out, float
                    reinterpret_cast<float*>(w + L.s_fold), out, lse, qm, vmean, d, Nk_pad, o_strides,
                    causal, sm_scale, dtype, qk_mode | flags, status, stream, who,
                    reinterpret_cast<unsigned*>(status) + 3, pk,
-                   (L.total > L.base_total && workspace_bytes >= L.total) ? w + L.part : nullptr);
+                   (L.total > L.base_total && workspace_bytes >= L.total) ? w + L.part : nullptr, status_host);
 }
 
 }  // namespace
@@ -345,6 +347,19 @@ int sage_attn_fwd_ex(const void* q8, const float* sq, const void* k8, const floa
                    causal, sm_scale, out_dtype, qk_mode, status, stream, "sage_attn_fwd_ex");
 }
 
+int sage_attn_fwd_reported(const void* q8, const float* sq, const void* k8, const float* sk,
+                           const void* v8t, const float* svp, const float* s_fold, void* out,
+                           float* lse, const float* qm, const float* vmean,
+                           int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int64_t Nk_pad, int64_t head_dim,
+                           const int64_t o_strides[3], int causal, float sm_scale, int out_dtype, int qk_mode,
+                           int32_t* status, int32_t* status_host, void* stream) {
+  if (reinterpret_cast<uintptr_t>(status_host) & 3u) return fail(SAGE_E_ARG, "sage_attn_fwd_reported: status_host must be 4-byte aligned");
+  const Dims d = {B, Hq, Hkv, Nq, Nk, head_dim};
+  return attn_impl(q8, sq, k8, sk, v8t, svp, s_fold, out, lse, qm, vmean, d, Nk_pad, o_strides,
+                   causal, sm_scale, out_dtype, qk_mode, status, stream, "sage_attn_fwd_reported", nullptr, kNotPacked, nullptr,
+                   status_host);
+}
+
 int sage_status_mirror(const int32_t* status_dev, int32_t* status_host, int words, void* stream) {
   g_err[0] = 0;
   if (!status_dev || !status_host) return fail(SAGE_E_ARG, "sage_status_mirror: null pointer argument");
@@ -420,14 +435,27 @@ int sage_attention_ex(const void* q, const void* k, const void* v, void* out, fl
                         o_strides, dtype, qk_mode, causal, smooth_k, smooth_v, sm_scale, stream, "sage_attention_ex");
 }
 
-int sage_attention_varlen(const void* q, const void* k, const void* v, void* out,
+int sage_attention_reported(const void* q, const void* k, const void* v, void* out, float* lse,
+                            void* workspace, size_t workspace_bytes,
+                            int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int64_t head_dim,
+                            const int64_t q_strides[3], const int64_t k_strides[3],
+                            const int64_t v_strides[3], const int64_t o_strides[3],
+                            int dtype, int qk_mode, int causal, int smooth_k, int smooth_v, float sm_scale,
+                            int32_t* status_host, void* stream) {
+  const Dims d = {B, Hq, Hkv, Nq, Nk, head_dim};
+  return attention_impl(q, k, v, out, lse, workspace, workspace_bytes, d, q_strides, k_strides, v_strides,
+                        o_strides, dtype, qk_mode, causal, smooth_k, smooth_v, sm_scale, stream, "sage_attention_reported",
+                        status_host);
+}
+
+int sage_attention_varlen_reported(const void* q, const void* k, const void* v, void* out,
                           const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
                           void* workspace, size_t workspace_bytes,
                           int64_t n_seq, int64_t Hq, int64_t Hkv,
                           int64_t total_q, int64_t total_k, int64_t max_q, int64_t max_k, int64_t head_dim,
                           const int64_t q_strides[2], const int64_t k_strides[2],
                           const int64_t v_strides[2], const int64_t o_strides[2],
-                          int dtype, int qk_mode, int causal, int smooth_k, float sm_scale, void* stream) {
+                          int dtype, int qk_mode, int causal, int smooth_k, float sm_scale, int32_t* status_host, void* stream) {
   g_err[0] = 0;
   if (!cu_seqlens_q || !cu_seqlens_k) return fail(SAGE_E_ARG, "sage_attention_varlen: cu_seqlens pointer is null");
   if ((reinterpret_cast<uintptr_t>(cu_seqlens_q) | reinterpret_cast<uintptr_t>(cu_seqlens_k)) & 3u)
@@ -444,7 +472,20 @@ int sage_attention_varlen(const void* q, const void* k, const void* v, void* out
   const Dims d = {n_seq, Hq, Hkv, max_q, max_k, head_dim};
   const Packed pk = {cu_seqlens_q, cu_seqlens_k, total_q, total_k, nullptr, 0};
   return attention_impl(q, k, v, out, nullptr, workspace, workspace_bytes, d, qs, ks, vs, os, dtype, qk_mode,
-                        causal, smooth_k, 0, sm_scale, stream, "sage_attention_varlen", pk);
+                        causal, smooth_k, 0, sm_scale, stream, "sage_attention_varlen", status_host, pk);
+}
+
+int sage_attention_varlen(const void* q, const void* k, const void* v, void* out,
+                          const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
+                          void* workspace, size_t workspace_bytes,
+                          int64_t n_seq, int64_t Hq, int64_t Hkv,
+                          int64_t total_q, int64_t total_k, int64_t max_q, int64_t max_k, int64_t head_dim,
+                          const int64_t q_strides[2], const int64_t k_strides[2],
+                          const int64_t v_strides[2], const int64_t o_strides[2],
+                          int dtype, int qk_mode, int causal, int smooth_k, float sm_scale, void* stream) {
+  return sage_attention_varlen_reported(q, k, v, out, cu_seqlens_q, cu_seqlens_k, workspace, workspace_bytes, n_seq, Hq, Hkv,
+                                        total_q, total_k, max_q, max_k, head_dim, q_strides, k_strides, v_strides, o_strides,
+                                        dtype, qk_mode, causal, smooth_k, sm_scale, nullptr, stream);
 }
 
 }  // extern "C"

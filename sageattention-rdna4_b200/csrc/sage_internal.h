@@ -57,6 +57,7 @@ struct AttnParams {
   unsigned* skipped;                                   // optional: (warp, key tile) pairs the fast path skipped
   const int32_t *cu_q, *cu_k;                          // packed variable-length batch (see PrologueParams); null otherwise
   int64_t Tq, Tk;                                      // with cu_q / cu_k: tokens in the packed tensors
+  int32_t* status_host;                                // optional, pinned host memory: receives the status word of a call that failed
   const int* plan;                                     // packed batch, optional: the prologue's work list
   void* part;                                          // optional: split_scratch_bytes() of scratch; without it the keys of a call are not split
 };

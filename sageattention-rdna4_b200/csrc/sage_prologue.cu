@@ -247,8 +247,6 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   extern __shared__ uint8_t qt_smem[];
   __shared__ long long s_item[QT_STAGES];
   __shared__ int s_plan[VARLEN ? 4 * (PLAN_MAX_SEQS + 1) : 1];
-  wait_for_predecessor();            // the means and the cleared control block
-  allow_successor();                 // persistent grid: every CTA is resident
   constexpr float QMAX = INT8 ? I8_MAX : F8_MAX;
   constexpr int QDIV = INT8 ? 127 : 448;
 
@@ -257,6 +255,14 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint8_t* gbase = qt_smem + (base - raw_addr);
   const uint32_t bar0 = base + QT_STAGES * QT_STAGE_BYTES;
   const int tid = threadIdx.x, c = tid & 7, r0 = tid >> 3, lane = tid & 31, warp = tid >> 5;
+
+  if (tid == 0) {
+    for (int s = 0; s < QT_STAGES; ++s)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8u * (uint32_t)s), "r"(1u) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  wait_for_predecessor();            // the means and the cleared control block
+  allow_successor();                 // persistent grid: every CTA is resident
 
   const long long tiles_q = (a.Nq + TILE - 1) / TILE, tiles_k = a.N_pad / TILE;
   const long long items_k = a.BHkv * tiles_k, items_q = a.BHq * tiles_q;
@@ -352,11 +358,6 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"((int)row), "r"(h), "r"(b) : "memory");
   };
 
-  if (tid == 0) {
-    for (int s = 0; s < QT_STAGES; ++s)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8u * (uint32_t)s), "r"(1u) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
   __syncthreads();
   long long drawn = 0;
   if (tid == 0) {

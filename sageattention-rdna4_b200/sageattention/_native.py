@@ -54,6 +54,16 @@ SIGNATURES = {
                                              _I64, _I64, _I64, _I64, _I64, _I64, _I64, _I64,
                                              _S3, _S3, _S3, _S3, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                              ctypes.c_int, ctypes.c_float, _P]),
+    "sage_attention_reported": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, ctypes.c_size_t, _I64, _I64, _I64, _I64, _I64, _I64,
+                                               _S3, _S3, _S3, _S3, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                               ctypes.c_int, ctypes.c_int, ctypes.c_float, _P, _P]),
+    "sage_attention_varlen_reported": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, ctypes.c_size_t,
+                                                      _I64, _I64, _I64, _I64, _I64, _I64, _I64, _I64,
+                                                      _S3, _S3, _S3, _S3, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                                      ctypes.c_int, ctypes.c_float, _P, _P]),
+    "sage_attn_fwd_reported": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P,
+                                              _I64, _I64, _I64, _I64, _I64, _I64, _I64, _S3,
+                                              ctypes.c_int, ctypes.c_float, ctypes.c_int, ctypes.c_int, _P, _P, _P]),
     "sage_status_mirror": (ctypes.c_int, [_P, _P, ctypes.c_int, _P]),
     "sage_debug_tiles_per_cta": (None, [ctypes.c_int]),
     "sage_debug_skip_threshold": (None, [ctypes.c_float]),

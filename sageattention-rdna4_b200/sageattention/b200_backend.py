@@ -222,11 +222,12 @@ def attn_launch(pq: Dict[str, torch.Tensor], out: torch.Tensor, is_causal: bool,
 # code in the call's status word (a word of the workspace) and the output of that call is
 # undefined.  The reference raises in such a case only in its strict mode and otherwise falls back
 # (sageattention/sk1_backend/__init__.py:1022-1027,1114-1123); this path has no fallback, so the
-# failure must reach the caller.  After every call a 4-byte copy of the status word into pinned
-# host memory is enqueued behind it (no synchronisation); the next call on that stream, `check()`
-# or `status()` looks at the host word and raises RuntimeError when it is non-zero.
+# failure must reach the caller.  The attention kernel of a call that failed writes the status word
+# into a word of pinned host memory (one that succeeds writes nothing, so nothing follows a call on
+# the stream); the next call on that stream, `check()` or `status()` looks at the host word and
+# raises RuntimeError when it is non-zero.
 # SAGEATTN_B200_STRICT=1 synchronises after every call and checks at once;
-# SAGEATTN_B200_WATCH=0 switches the copy off.
+# SAGEATTN_B200_WATCH=0 switches the report off.
 STATUS_BITS = ((1, "the TMA producer of the attention kernel"), (2, "the MMA issuer of the attention kernel"),
                (4, "a softmax warp of the attention kernel"), (8, "a tile load of the quantisation prologue"))
 
@@ -250,7 +251,7 @@ def _env_flag(name: str, default: bool) -> bool:
 # exponentiated, which on inputs with a few dominant keys removes most of the softmax work; on
 # inputs without such keys the tests only cost (3 to 6 %).  The kernels count what they skip, so
 # the choice is made from evidence: a call signature (shape, mask, dtype) starts with the tests
-# on; one such call is a probe whose count comes back to the host with the status mirror (no
+# on; one such call is a probe whose count comes back to the host in a small copy (no
 # synchronisation: the result is picked up by a later call once its event has completed); a probe
 # that skipped less than PROBE_MIN_SHARE of the (warp, key tile) pairs sends the next PLAIN_CALLS
 # calls of that signature to the kernels without the tests, after which the next call probes
@@ -297,7 +298,7 @@ class _Adaptive:
 class _StreamState:
     """What the path keeps per (device, stream): one grow-only workspace (intermediates of a call
     live only until its attention kernel has run, and calls on one stream are ordered) and the
-    pinned host word that mirrors the status word of the most recent call."""
+    pinned host word that receives the status word of a call that failed."""
 
     __slots__ = ("ws", "host", "host_word", "status_off", "shape", "adaptive", "probe_host", "last_share")
 
@@ -367,6 +368,17 @@ def _host_word(st: _StreamState):
         st.host = torch.zeros((1,), dtype=torch.int32).pin_memory()
         st.host_word = ctypes.c_int32.from_address(st.host.data_ptr())
     return st.host_word
+
+
+def _report_to(st: _StreamState, capturing: bool) -> int:
+    """Address of the host word a failing call reports to, 0 for none.  (Pinned memory is not
+    allocated under capture: a first call that is captured does not report.)"""
+    if st.host is not None:
+        return st.host.data_ptr() if _WATCH else 0
+    if not _WATCH or capturing or st.host_word is not None:
+        return 0
+    _host_word(st)
+    return st.host.data_ptr()
 
 
 def clear_workspaces():
@@ -509,16 +521,13 @@ def sage_call(q, k, v, tensor_layout="HND", is_causal=False, sm_scale=None, smoo
         qk_mode = -_native.SAGE_QK_NO_FAST_PATH if qk_mode < 0 else (qk_mode | _native.SAGE_QK_NO_FAST_PATH)
     args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 0 if lse is None else lse.data_ptr(),
             ws_ptr, ws.numel(), b, h, hkv, n, nk, d, q3, k3, v3, o3, dt, qk_mode,
-            1 if is_causal else 0, 1 if smooth_k else 0, 1 if smooth_v else 0, scale, stream_id)
-    watch = _WATCH and not (capturing and st.host_word is None)
+            1 if is_causal else 0, 1 if smooth_k else 0, 1 if smooth_v else 0, scale, _report_to(st, capturing), stream_id)
     same_dev = torch.cuda.current_device() == dev.index
     if not same_dev:
         prev_dev = torch.cuda.current_device()
         torch.cuda.set_device(dev)
     try:
-        rc = lib.sage_attention_ex(*args)
-        if watch and not rc:
-            rc = lib.sage_status_mirror(ws_ptr + status_off, ctypes.addressof(_host_word(st)), 1, stream_id)
+        rc = lib.sage_attention_reported(*args)
         if probe and not rc:
             if st.probe_host is None:
                 st.probe_host = torch.zeros((4,), dtype=torch.int32).pin_memory()
@@ -620,16 +629,14 @@ def sage_call_varlen(q, k, v, cu_q, cu_k, max_q: int, max_k: int, is_causal=Fals
         ws = _grow(st, dev, ws_bytes)
     st.status_off, st.shape = status_off, (n_seq, hq, hkv, max_q, max_k)
     capturing = torch.cuda.is_current_stream_capturing()
-    watch = _WATCH and not (capturing and st.host_word is None)
     args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_q.data_ptr(), cu_k.data_ptr(),
             ws.data_ptr(), ws.numel(), n_seq, hq, hkv, tq, tk, max_q, max_k, d,
             _native.strides2(q.stride(0), q.stride(1)), _native.strides2(k.stride(0), k.stride(1)),
             _native.strides2(v.stride(0), v.stride(1)), _native.strides2(out.stride(0), out.stride(1)),
-            _dtype_code(q.dtype), -1, 1 if is_causal else 0, 1 if smooth_k else 0, scale, stream_id)
+            _dtype_code(q.dtype), -1, 1 if is_causal else 0, 1 if smooth_k else 0, scale,
+            _report_to(st, capturing), stream_id)
     with torch.cuda.device(dev):
-        rc = lib.sage_attention_varlen(*args)
-        if watch and not rc:
-            rc = lib.sage_status_mirror(ws.data_ptr() + status_off, ctypes.addressof(_host_word(st)), 1, stream_id)
+        rc = lib.sage_attention_varlen_reported(*args)
     if rc:
         _native.check(rc, "sage_attention_varlen")
     if _STRICT:
