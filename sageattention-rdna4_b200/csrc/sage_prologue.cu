@@ -183,6 +183,8 @@ struct QuantArgs {
   long long Tq, Tk;               // VARLEN kernels: tokens in the packed q and k/v tensors
   const int* plan;                // VARLEN kernels, optional: the work list of plan_packed_kernel
   int n_seq;
+  int only_q;                     // the K and V tiles are done (quant_short_kernel): Q tiles only
+  long long drawn;                // items the work counter starts from: those that are done
 };
 
 // rn(x / s) given rc = rn(1/s)
@@ -236,6 +238,209 @@ __device__ __forceinline__ uint32_t i8x4_magic2(float2 ab, float2 cd) {
                      __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x0040), 0x5410);
 }
 
+// ------------------------------------------------------------------------------------------------
+// One 128-token tile, already in shared memory (128 rows of 256 bytes), by 256 threads.  Thread
+// (c = tid & 7, r0 = tid >> 3) owns columns 8c..8c+7 and 64+8c..64+8c+7 of rows r0, r0+32, r0+64,
+// r0+96.  N: live tokens of the sequence.
+// ------------------------------------------------------------------------------------------------
+template <typename T, bool INT8>
+__device__ __forceinline__ void quant_q_tile(const QuantArgs& a, const uint8_t* st, long long bh, long long n_base,
+                                             long long N, int c, int r0) {
+  constexpr float QMAX = INT8 ? I8_MAX : F8_MAX;
+  constexpr int QDIV = INT8 ? 127 : 448;
+  float mu[16];
+  if (a.qm != nullptr) {
+    const long long b = bh / a.Hq, h = bh - b * a.Hq, bh_kv = b * a.H + h / a.group;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) { mu[e] = a.mean[(size_t)bh_kv * HD + 8 * c + e]; mu[8 + e] = a.mean[(size_t)bh_kv * HD + 64 + 8 * c + e]; }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = r0 + 32 * i;
+    const long long nrow = n_base + t;
+    float x[16];
+    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
+    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
+    float amax = 0.f;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) amax = fmaxf(amax, fabsf(x[e]));
+    amax = fmaxf(quarter_warp_max(amax), SCALE_FLOOR);
+    const float qinv = __fdiv_rn(QMAX, amax);
+    float2 y[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) y[e] = make_float2(__fmul_rn(x[2 * e], qinv), __fmul_rn(x[2 * e + 1], qinv));
+    uint2 w0, w1;
+    if (INT8) {
+      w0.x = i8x4_magic2(y[0], y[1]); w0.y = i8x4_magic2(y[2], y[3]);
+      w1.x = i8x4_magic2(y[4], y[5]); w1.y = i8x4_magic2(y[6], y[7]);
+    } else {
+      w0.x = e4m3x4(y[0].x, y[0].y, y[1].x, y[1].y); w0.y = e4m3x4(y[2].x, y[2].y, y[3].x, y[3].y);
+      w1.x = e4m3x4(y[4].x, y[4].y, y[5].x, y[5].y); w1.y = e4m3x4(y[6].x, y[6].y, y[7].x, y[7].y);
+    }
+    if (nrow < N) {
+      uint8_t* dst = a.q8 + ((size_t)bh * a.Nq + nrow) * HD + 8 * c;
+      *reinterpret_cast<uint2*>(dst) = w0;
+      *reinterpret_cast<uint2*>(dst + 64) = w1;
+      if (c == 0) a.sq[(size_t)bh * a.Nq + nrow] = div_const<QDIV>(amax);
+    }
+    if (a.qm != nullptr) {                          // fixed-order fp32 dot product of the raw row
+      float d = 0.f;
+#pragma unroll
+      for (int e = 0; e < 16; ++e) d = __fmaf_rn(x[e], mu[e], d);
+      d += __shfl_xor_sync(0xffffffffu, d, 4);
+      d += __shfl_xor_sync(0xffffffffu, d, 2);
+      d += __shfl_xor_sync(0xffffffffu, d, 1);
+      if (c == 0 && nrow < N) a.qm[(size_t)bh * a.Nq + nrow] = d;
+    }
+  }
+}
+
+// mu: mean of K per column (read when a.sub_mean)
+template <typename T, bool INT8>
+__device__ __forceinline__ void quant_k_tile(const QuantArgs& a, const uint8_t* st, const float* mu, long long bh,
+                                             long long n_base, long long N, int c, int r0) {
+  constexpr int QDIV = INT8 ? 127 : 448;
+  const long long N_pad = a.N_pad;
+  float2 nmu[8];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float* m0 = mu + 8 * c + 2 * e;
+    nmu[e] = a.sub_mean ? make_float2(-m0[0], -m0[1]) : make_float2(0.f, 0.f);
+    nmu[4 + e] = a.sub_mean ? make_float2(-m0[64], -m0[65]) : make_float2(0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = r0 + 32 * i;
+    const long long nrow = n_base + t;
+    const bool live = nrow < N;
+    float x[16];
+    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
+    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
+    float2 xs[8];
+    float amax = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      xs[e] = __fadd2_rn(make_float2(x[2 * e], x[2 * e + 1]), nmu[e]);
+      amax = fmaxf(amax, fmaxf(fabsf(xs[e].x), fabsf(xs[e].y)));
+    }
+    amax = quarter_warp_max(live ? amax : 0.f);
+    const float sk = fmaxf(div_const<QDIV>(amax), SCALE_FLOOR);
+    const float rc = __frcp_rn(sk);
+    uint2 w0, w1;
+    if (INT8) {
+      // the sign of a zero quotient does not reach an int8 code, so the packed form is enough
+      const float2 rc2 = make_float2(rc, rc), ns2 = make_float2(-sk, -sk);
+      float2 y[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float2 q0 = __fmul2_rn(xs[e], rc2);
+        const float2 r = __ffma2_rn(q0, ns2, xs[e]);
+        y[e] = __ffma2_rn(r, rc2, q0);
+      }
+      w0.x = i8x4_magic2(y[0], y[1]); w0.y = i8x4_magic2(y[2], y[3]);
+      w1.x = i8x4_magic2(y[4], y[5]); w1.y = i8x4_magic2(y[6], y[7]);
+    } else {
+      float y[16];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { y[2 * e] = div_by_scale(xs[e].x, sk, rc); y[2 * e + 1] = div_by_scale(xs[e].y, sk, rc); }
+      w0.x = e4m3x4(y[0], y[1], y[2], y[3]); w0.y = e4m3x4(y[4], y[5], y[6], y[7]);
+      w1.x = e4m3x4(y[8], y[9], y[10], y[11]); w1.y = e4m3x4(y[12], y[13], y[14], y[15]);
+    }
+    if (!live) { w0 = make_uint2(0u, 0u); w1 = w0; }
+    // rows are stored permuted inside 16-row blocks: key 4cc + jj of a block goes to row
+    // 2cc + jj (jj < 2) or 8 + 2cc + jj - 2, the order in which the attention kernel's
+    // 16-lane TMEM loads hand a thread four consecutive keys
+    const long long o16 = nrow & 15, srow = (nrow & ~15LL) | ((o16 & 2) ? 8 + 2 * (o16 >> 2) + (o16 & 1) : 2 * (o16 >> 2) + (o16 & 1));
+    uint8_t* dst = a.k8 + ((size_t)bh * N_pad + srow) * HD + 8 * c;
+    *reinterpret_cast<uint2*>(dst) = w0;
+    *reinterpret_cast<uint2*>(dst + 64) = w1;
+    if (c == 0) a.sk[(size_t)bh * N_pad + nrow] = live ? sk : 1.0f;
+  }
+}
+
+// The threads that share a tile: the whole block (BAR 0) or half of one (BAR 1 and 2).
+template <int BAR> __device__ __forceinline__ void tile_sync() { asm volatile("bar.sync %0, 256;" ::"n"(BAR) : "memory"); }
+
+// vmean: mean of V per column, or null.  The tile's scales also go to sv_tile, if given.  The stage is
+// overwritten with the codes.  Returns this thread's largest scale of a live row.
+template <typename T, bool VARLEN, int BAR>
+__device__ __forceinline__ float quant_v_tile(const QuantArgs& a, uint8_t* st, const float* vmean, float* sv_tile, long long bh,
+                                              long long n_base, long long N, int tid) {
+  const int c = tid & 7, r0 = tid >> 3, lane = tid & 31, warp = tid >> 5;
+  const long long N_pad = a.N_pad;
+  float vmu[16];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    vmu[e] = vmean ? vmean[8 * c + e] : 0.f;
+    vmu[8 + e] = vmean ? vmean[64 + 8 * c + e] : 0.f;
+  }
+  float svmax = 0.f;
+  uint2 w0[4], w1[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = r0 + 32 * i;
+    const long long nrow = n_base + t;
+    const bool live = nrow < N;
+    float x[16];
+    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
+    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
+    float amax = 0.f;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      if (vmean) x[e] = live ? __fsub_rn(x[e], vmu[e]) : 0.f;
+      if (VARLEN && !live) x[e] = 0.f;               // the rows behind a packed sequence are its neighbour's
+      amax = fmaxf(amax, fabsf(x[e]));
+    }
+    amax = quarter_warp_max(amax);
+    const float sv = fmaxf(div_const<448>(amax), SCALE_FLOOR);
+    const float rc = __frcp_rn(sv);
+    float y[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) y[e] = div_by_scale(x[e], sv, rc);
+    w0[i].x = e4m3x4(y[0], y[1], y[2], y[3]); w0[i].y = e4m3x4(y[4], y[5], y[6], y[7]);
+    w1[i].x = e4m3x4(y[8], y[9], y[10], y[11]); w1[i].y = e4m3x4(y[12], y[13], y[14], y[15]);
+    if (c == 0) {
+      a.sv[(size_t)bh * N_pad + nrow] = live ? sv : 0.0f;
+      if (sv_tile) sv_tile[t] = live ? sv : 0.0f;
+      if (live) svmax = fmaxf(svmax, sv);
+    }
+  }
+  tile_sync<BAR>();                // every thread has read its rows: the stage becomes the code tile
+  uint32_t* vt = reinterpret_cast<uint32_t*>(st);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int t = r0 + 32 * i;
+    const int key = (((t >> 4) & 7) << 2) ^ ((t & 1) << 4);
+    *reinterpret_cast<uint2*>(&vt[t * 32 + ((2 * c) ^ key)]) = w0[i];
+    *reinterpret_cast<uint2*>(&vt[t * 32 + ((16 + 2 * c) ^ key)]) = w1[i];
+  }
+  tile_sync<BAR>();
+  {
+    const int tg = lane & 7, dq = 4 * warp + (lane >> 3);
+    uint32_t o[4][4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int tk = 16 * tg + 4 * g;
+      const uint32_t w0_ = vt[(tk + 0) * 32 + (dq ^ (tg << 2))];
+      const uint32_t w1_ = vt[(tk + 1) * 32 + (dq ^ (tg << 2) ^ 16)];
+      const uint32_t w2_ = vt[(tk + 2) * 32 + (dq ^ (tg << 2))];
+      const uint32_t w3_ = vt[(tk + 3) * 32 + (dq ^ (tg << 2) ^ 16)];
+      const uint32_t t0 = __byte_perm(w0_, w1_, 0x5140), t1 = __byte_perm(w2_, w3_, 0x5140);
+      const uint32_t t2 = __byte_perm(w0_, w1_, 0x7362), t3 = __byte_perm(w2_, w3_, 0x7362);
+      o[0][g] = __byte_perm(t0, t1, 0x5410);
+      o[1][g] = __byte_perm(t0, t1, 0x7632);
+      o[2][g] = __byte_perm(t2, t3, 0x5410);
+      o[3][g] = __byte_perm(t2, t3, 0x7632);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      uint8_t* dst = a.v8t + ((size_t)bh * HD + 4 * dq + e) * N_pad + n_base + 16 * tg;
+      *reinterpret_cast<uint4*>(dst) = make_uint4(o[e][0], o[e][1], o[e][2], o[e][3]);
+    }
+  }
+  return svmax;
+}
+
 // VARLEN: a packed batch.  N, N_pad and Nq are then the capacity of a sequence's slot in the outputs
 // (sized for the longest sequence allowed); every sequence has its own length and its own first
 // token in the inputs, read from cu_q / cu_k.  Tiles past a sequence's end are neither loaded nor
@@ -247,9 +452,6 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   extern __shared__ uint8_t qt_smem[];
   __shared__ long long s_item[QT_STAGES];
   __shared__ int s_plan[VARLEN ? 4 * (PLAN_MAX_SEQS + 1) : 1];
-  constexpr float QMAX = INT8 ? I8_MAX : F8_MAX;
-  constexpr int QDIV = INT8 ? 127 : 448;
-
   const uint32_t raw_addr = qt_smem_u32(qt_smem);
   const uint32_t base = (raw_addr + 127u) & ~127u;
   uint8_t* gbase = qt_smem + (base - raw_addr);
@@ -265,9 +467,9 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   allow_successor();                 // persistent grid: every CTA is resident
 
   const long long tiles_q = (a.Nq + TILE - 1) / TILE, tiles_k = a.N_pad / TILE;
-  const long long items_k = a.BHkv * tiles_k, items_q = a.BHq * tiles_q;
+  const long long items_k = a.only_q ? 0 : a.BHkv * tiles_k, items_q = a.BHq * tiles_q;
   const long long fold_per_head = (a.N_pad + FOLD_KEYS - 1) / FOLD_KEYS;
-  const long long items_f = a.BHkv * fold_per_head;
+  const long long items_f = a.only_q ? 0 : a.BHkv * fold_per_head;
   const bool planned = VARLEN && a.plan != nullptr;
   const int P1 = VARLEN ? a.n_seq + 1 : 0;
   if (planned) {
@@ -319,7 +521,7 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   // simply takes fewer of them.  Thread 0 publishes the item of a stage in s_item and starts its
   // load; past the end it publishes -1 and completes the stage's barrier by hand.  The counter is
   // drawn one item ahead, so the atomic's round trip is off the critical path.
-  auto draw = [&]() { return (long long)atomicAdd(a.next_item, 1ULL); };
+  auto draw = [&]() { return (long long)atomicAdd(a.next_item, 1ULL) - a.drawn; };
   auto issue = [&](int stage, long long it) {
     const uint32_t bar_ = bar0 + 8u * (uint32_t)stage;
     if (it >= total) {
@@ -405,181 +607,16 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     } else if (which == 0) {
       // ---------------------------------- Q ----------------------------------
       const long long N = VARLEN ? seq_len : a.Nq;
-      float mu[16];
-      if (a.qm != nullptr) {
-        const long long b = bh / a.Hq, h = bh - b * a.Hq, bh_kv = b * a.H + h / a.group;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) { mu[e] = a.mean[(size_t)bh_kv * HD + 8 * c + e]; mu[8 + e] = a.mean[(size_t)bh_kv * HD + 64 + 8 * c + e]; }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = r0 + 32 * i;
-        const long long nrow = n_base + t;
-        float x[16];
-        unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
-        unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
-        float amax = 0.f;
-#pragma unroll
-        for (int e = 0; e < 16; ++e) amax = fmaxf(amax, fabsf(x[e]));
-        amax = fmaxf(quarter_warp_max(amax), SCALE_FLOOR);
-        const float qinv = __fdiv_rn(QMAX, amax);
-        float2 y[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) y[e] = make_float2(__fmul_rn(x[2 * e], qinv), __fmul_rn(x[2 * e + 1], qinv));
-        uint2 w0, w1;
-        if (INT8) {
-          w0.x = i8x4_magic2(y[0], y[1]); w0.y = i8x4_magic2(y[2], y[3]);
-          w1.x = i8x4_magic2(y[4], y[5]); w1.y = i8x4_magic2(y[6], y[7]);
-        } else {
-          w0.x = e4m3x4(y[0].x, y[0].y, y[1].x, y[1].y); w0.y = e4m3x4(y[2].x, y[2].y, y[3].x, y[3].y);
-          w1.x = e4m3x4(y[4].x, y[4].y, y[5].x, y[5].y); w1.y = e4m3x4(y[6].x, y[6].y, y[7].x, y[7].y);
-        }
-        if (nrow < N) {
-          uint8_t* dst = a.q8 + ((size_t)bh * a.Nq + nrow) * HD + 8 * c;
-          *reinterpret_cast<uint2*>(dst) = w0;
-          *reinterpret_cast<uint2*>(dst + 64) = w1;
-          if (c == 0) a.sq[(size_t)bh * a.Nq + nrow] = div_const<QDIV>(amax);
-        }
-        if (a.qm != nullptr) {                          // fixed-order fp32 dot product of the raw row
-          float d = 0.f;
-#pragma unroll
-          for (int e = 0; e < 16; ++e) d = __fmaf_rn(x[e], mu[e], d);
-          d += __shfl_xor_sync(0xffffffffu, d, 4);
-          d += __shfl_xor_sync(0xffffffffu, d, 2);
-          d += __shfl_xor_sync(0xffffffffu, d, 1);
-          if (c == 0 && nrow < N) a.qm[(size_t)bh * a.Nq + nrow] = d;
-        }
-      }
+      quant_q_tile<T, INT8>(a, st, bh, n_base, N, c, r0);
     } else if (which == 1) {
       // ---------------------------------- K ----------------------------------
-      const long long N = VARLEN ? seq_len : a.N, N_pad = a.N_pad;
-      float2 nmu[8];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float* m0 = a.mean + (size_t)bh * HD + 8 * c + 2 * e;
-        nmu[e] = a.sub_mean ? make_float2(-m0[0], -m0[1]) : make_float2(0.f, 0.f);
-        nmu[4 + e] = a.sub_mean ? make_float2(-m0[64], -m0[65]) : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = r0 + 32 * i;
-        const long long nrow = n_base + t;
-        const bool live = nrow < N;
-        float x[16];
-        unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
-        unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
-        float2 xs[8];
-        float amax = 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          xs[e] = __fadd2_rn(make_float2(x[2 * e], x[2 * e + 1]), nmu[e]);
-          amax = fmaxf(amax, fmaxf(fabsf(xs[e].x), fabsf(xs[e].y)));
-        }
-        amax = quarter_warp_max(live ? amax : 0.f);
-        const float sk = fmaxf(div_const<QDIV>(amax), SCALE_FLOOR);
-        const float rc = __frcp_rn(sk);
-        uint2 w0, w1;
-        if (INT8) {
-          // the sign of a zero quotient does not reach an int8 code, so the packed form is enough
-          const float2 rc2 = make_float2(rc, rc), ns2 = make_float2(-sk, -sk);
-          float2 y[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float2 q0 = __fmul2_rn(xs[e], rc2);
-            const float2 r = __ffma2_rn(q0, ns2, xs[e]);
-            y[e] = __ffma2_rn(r, rc2, q0);
-          }
-          w0.x = i8x4_magic2(y[0], y[1]); w0.y = i8x4_magic2(y[2], y[3]);
-          w1.x = i8x4_magic2(y[4], y[5]); w1.y = i8x4_magic2(y[6], y[7]);
-        } else {
-          float y[16];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) { y[2 * e] = div_by_scale(xs[e].x, sk, rc); y[2 * e + 1] = div_by_scale(xs[e].y, sk, rc); }
-          w0.x = e4m3x4(y[0], y[1], y[2], y[3]); w0.y = e4m3x4(y[4], y[5], y[6], y[7]);
-          w1.x = e4m3x4(y[8], y[9], y[10], y[11]); w1.y = e4m3x4(y[12], y[13], y[14], y[15]);
-        }
-        if (!live) { w0 = make_uint2(0u, 0u); w1 = w0; }
-        // rows are stored permuted inside 16-row blocks: key 4cc + jj of a block goes to row
-        // 2cc + jj (jj < 2) or 8 + 2cc + jj - 2, the order in which the attention kernel's
-        // 16-lane TMEM loads hand a thread four consecutive keys
-        const long long o16 = nrow & 15, srow = (nrow & ~15LL) | ((o16 & 2) ? 8 + 2 * (o16 >> 2) + (o16 & 1) : 2 * (o16 >> 2) + (o16 & 1));
-        uint8_t* dst = a.k8 + ((size_t)bh * N_pad + srow) * HD + 8 * c;
-        *reinterpret_cast<uint2*>(dst) = w0;
-        *reinterpret_cast<uint2*>(dst + 64) = w1;
-        if (c == 0) a.sk[(size_t)bh * N_pad + nrow] = live ? sk : 1.0f;
-      }
+      const long long N = VARLEN ? seq_len : a.N;
+      quant_k_tile<T, INT8>(a, st, a.mean + (size_t)bh * HD, bh, n_base, N, c, r0);
     } else if (which == 2) {
       // ---------------------------------- V ----------------------------------
-      const long long N = VARLEN ? seq_len : a.N, N_pad = a.N_pad;
-      float vmu[16];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        vmu[e] = a.vmean ? a.vmean[(size_t)bh * HD + 8 * c + e] : 0.f;
-        vmu[8 + e] = a.vmean ? a.vmean[(size_t)bh * HD + 64 + 8 * c + e] : 0.f;
-      }
-      float svmax = 0.f;
-      uint2 w0[4], w1[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = r0 + 32 * i;
-        const long long nrow = n_base + t;
-        const bool live = nrow < N;
-        float x[16];
-        unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
-        unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
-        float amax = 0.f;
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          if (a.vmean) x[e] = live ? __fsub_rn(x[e], vmu[e]) : 0.f;
-          if (VARLEN && !live) x[e] = 0.f;               // the rows behind a packed sequence are its neighbour's
-          amax = fmaxf(amax, fabsf(x[e]));
-        }
-        amax = quarter_warp_max(amax);
-        const float sv = fmaxf(div_const<448>(amax), SCALE_FLOOR);
-        const float rc = __frcp_rn(sv);
-        float y[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) y[e] = div_by_scale(x[e], sv, rc);
-        w0[i].x = e4m3x4(y[0], y[1], y[2], y[3]); w0[i].y = e4m3x4(y[4], y[5], y[6], y[7]);
-        w1[i].x = e4m3x4(y[8], y[9], y[10], y[11]); w1[i].y = e4m3x4(y[12], y[13], y[14], y[15]);
-        if (c == 0) {
-          a.sv[(size_t)bh * N_pad + nrow] = live ? sv : 0.0f;
-          if (live) svmax = fmaxf(svmax, sv);
-        }
-      }
-      __syncthreads();                 // every thread has read its rows: the stage becomes the code tile
-      uint32_t* vt = reinterpret_cast<uint32_t*>(gbase + (size_t)stage * QT_STAGE_BYTES);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = r0 + 32 * i;
-        const int key = (((t >> 4) & 7) << 2) ^ ((t & 1) << 4);
-        *reinterpret_cast<uint2*>(&vt[t * 32 + ((2 * c) ^ key)]) = w0[i];
-        *reinterpret_cast<uint2*>(&vt[t * 32 + ((16 + 2 * c) ^ key)]) = w1[i];
-      }
-      __syncthreads();
-      {
-        const int tg = lane & 7, dq = 4 * warp + (lane >> 3);
-        uint32_t o[4][4];
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int tk = 16 * tg + 4 * g;
-          const uint32_t w0_ = vt[(tk + 0) * 32 + (dq ^ (tg << 2))];
-          const uint32_t w1_ = vt[(tk + 1) * 32 + (dq ^ (tg << 2) ^ 16)];
-          const uint32_t w2_ = vt[(tk + 2) * 32 + (dq ^ (tg << 2))];
-          const uint32_t w3_ = vt[(tk + 3) * 32 + (dq ^ (tg << 2) ^ 16)];
-          const uint32_t t0 = __byte_perm(w0_, w1_, 0x5140), t1 = __byte_perm(w2_, w3_, 0x5140);
-          const uint32_t t2 = __byte_perm(w0_, w1_, 0x7362), t3 = __byte_perm(w2_, w3_, 0x7362);
-          o[0][g] = __byte_perm(t0, t1, 0x5410);
-          o[1][g] = __byte_perm(t0, t1, 0x7632);
-          o[2][g] = __byte_perm(t2, t3, 0x5410);
-          o[3][g] = __byte_perm(t2, t3, 0x7632);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          uint8_t* dst = a.v8t + ((size_t)bh * HD + 4 * dq + e) * N_pad + n_base + 16 * tg;
-          *reinterpret_cast<uint4*>(dst) = make_uint4(o[e][0], o[e][1], o[e][2], o[e][3]);
-        }
-      }
+      const long long N = VARLEN ? seq_len : a.N;
+      float svmax = quant_v_tile<T, VARLEN, 0>(a, gbase + (size_t)stage * QT_STAGE_BYTES, a.vmean ? a.vmean + (size_t)bh * HD : nullptr,
+                                               nullptr, bh, n_base, N, tid);
       // per-head max of the V scale (all scales are >= 0, so the unsigned order of the bit patterns
       // is the float order); S and SVP are folded by the closing items of the list
 #pragma unroll
@@ -631,6 +668,180 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 }
 
 // ------------------------------------------------------------------------------------------------
+// Short key sequences (at most SHORT_CTAS tiles): the whole prologue in one launch.  The CTAs of a
+// cluster hold the K and V tiles of one K/V head in their shared memory, one of each per CTA.  Half of a CTA's threads sum the K tiles' columns, hand the sums to the other CTAs through
+// distributed shared memory, and quantise with the mean of all; the other half quantises V, and the
+// largest V scale of the cluster gives S.  K is read once, there are no control words to clear, no
+// work counter and no fold items: such calls spend their time on launches and round trips to
+// memory, not on bandwidth.  48 heads of 288 tokens: three launches of 17 us in all before, one of
+// 10 us now.
+// Further clusters take the Q tiles, one per half.
+// ------------------------------------------------------------------------------------------------
+struct ShortArgs {
+  float *mean, *vmean;
+  unsigned* words;                // control words, cleared here for the kernels behind this one
+  int n_words, kv_clusters;
+  int counter_word;               // the work counter, which is set to the number of tiles done here
+  unsigned items;
+  long long items_q;
+};
+constexpr int SHORT_CTAS = 16;    // the largest cluster, with two CTAs on an SM
+namespace short_smem {
+constexpr uint32_t RED = 2 * QT_STAGE_BYTES;                    // [2][4][128] fp64: column sums of warps
+constexpr uint32_t PART = RED + 2 * 4 * HD * 8;                 // [2][SHORT_CTAS][128] fp64: column sums of CTAs
+constexpr uint32_t MEAN = PART + 2 * SHORT_CTAS * HD * 8;       // [2][128] fp32
+constexpr uint32_t SV = MEAN + 2 * HD * 4;                      // [128] fp32: V scales
+constexpr uint32_t BARS = SV + TILE * 4;
+constexpr uint32_t SVMAX = BARS + 2 * 8;
+constexpr uint32_t BYTES = SVMAX + 16 + 128 /* alignment slack */;
+static_assert(2 * (BYTES + 1024) <= 228 * 1024, "two CTAs share an SM");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+template <typename T, bool INT8>
+__global__ void __launch_bounds__(512, 2)
+quant_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                   const __grid_constant__ CUtensorMap tm_v, const QuantArgs a, const ShortArgs sa) {
+  namespace L = short_smem;
+  extern __shared__ uint8_t qt_smem[];
+  const uint32_t raw_addr = qt_smem_u32(qt_smem), base = (raw_addr + 127u) & ~127u;
+  uint8_t* gbase = qt_smem + (base - raw_addr);
+  const int tid = threadIdx.x, grp = tid >> 8, gt = tid & 255, lane = tid & 31, gwarp = gt >> 5;
+  const int c = gt & 7, r0 = gt >> 3;
+  uint32_t C, rank;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(C));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int cluster = (int)(blockIdx.x / C);
+  const uint32_t bar = base + L::BARS + 8u * (uint32_t)grp;          // this half's tile
+  volatile unsigned* svmax_s = reinterpret_cast<volatile unsigned*>(gbase + L::SVMAX);
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(base + L::BARS + 8u * (uint32_t)i), "r"(1u) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *svmax_s = 0u;
+  }
+  __syncthreads();
+  cluster_arrive();
+  cluster_wait();                    // every CTA of the cluster runs: its shared memory may be written
+  wait_for_predecessor();            // an earlier call may still be using the buffers
+  allow_successor();
+  if (blockIdx.x == 0)
+    for (int i = tid; i < sa.n_words; i += 512) sa.words[i] = (i == sa.counter_word) ? sa.items : 0u;
+
+  auto load = [&](const CUtensorMap* map, long long tile, long long bh, long long heads) {
+    const uint32_t dst = base + (uint32_t)grp * QT_STAGE_BYTES;
+    const int b = (int)(bh / heads), h = (int)(bh - (long long)b * heads);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(QT_STAGE_BYTES) : "memory");
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"((int)(tile * TILE)), "r"(h), "r"(b) : "memory");
+  };
+  // bounded wait; a thread that gives up reports it and goes on, so that no barrier misses it
+  auto landed = [&]() {
+    if (qt_try_wait(bar, 0)) return;
+    const long long t0 = clock64();
+    while (!qt_try_wait(bar, 0))
+      if (clock64() - t0 > QT_WAIT_CYCLES) { atomicOr(a.status, 1); if (a.status2) atomicOr(a.status2, 8); return; }
+  };
+  uint8_t* stage = gbase + (uint32_t)grp * QT_STAGE_BYTES;
+  auto half_sync = [&]() { if (grp == 0) tile_sync<1>(); else tile_sync<2>(); };
+
+  if (cluster >= sa.kv_clusters) {   // Q tiles
+    const long long tiles_q = (a.Nq + TILE - 1) / TILE;
+    const long long item = ((long long)(cluster - sa.kv_clusters) * C + rank) * 2 + grp;
+    if (item >= sa.items_q) return;
+    const long long bh = item / tiles_q, tile = item - bh * tiles_q;
+    if (gt == 0) load(&tm_q, tile, bh, a.Hq);
+    landed();
+    quant_q_tile<T, INT8>(a, stage, bh, tile * TILE, a.Nq, c, r0);
+    return;
+  }
+
+  const long long bh = cluster, n_base = (long long)rank * TILE;      // tile `rank` of both tensors
+  if (gt == 0) load(grp == 0 ? &tm_k : &tm_v, rank, bh, a.H);
+  const bool has_mean = (grp == 0) ? a.sub_mean != 0 : sa.vmean != nullptr;
+  float* mean_s = reinterpret_cast<float*>(gbase + L::MEAN) + grp * HD;
+  if (has_mean) {
+    // column sums in fp64 (exact for fp16 values, see the top of the file): rows by half-warps,
+    // then warps, then CTAs, all in a fixed order
+    const int cc = gt & 15, rr = gt >> 4;
+    double acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.0;
+    landed();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      float x[8];
+      unpack8<T>(*reinterpret_cast<const uint4*>(stage + (rr + 16 * k) * 256 + 16 * cc), x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += (double)x[e];
+    }
+    double* red = reinterpret_cast<double*>(gbase + L::RED) + grp * 4 * HD + (gwarp & 3) * HD + 8 * cc;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], 16);
+    if (gwarp >= 4 && lane < 16)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) red[e] = acc[e];
+    half_sync();
+    if (gwarp < 4 && lane < 16)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) red[e] += acc[e];
+    half_sync();
+    if (gt < HD) {
+      const double* col = reinterpret_cast<const double*>(gbase + L::RED) + grp * 4 * HD + gt;
+      const double t = (col[0] + col[HD]) + (col[2 * HD] + col[3 * HD]);
+      const uint32_t at = base + L::PART + (uint32_t)((grp * SHORT_CTAS + rank) * HD + gt) * 8u;
+      for (uint32_t r = 0; r < C; ++r)
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(in_cta(at, r)), "d"(t) : "memory");
+    }
+  }
+  float svmax = 0.f;
+  float* sv_s = reinterpret_cast<float*>(gbase + L::SV);
+  auto quant_v = [&](const float* vmean) {
+    landed();
+    svmax = quant_v_tile<T, false, 2>(a, stage, vmean, sv_s, bh, n_base, a.N, gt);
+  };
+  cluster_arrive();                  // this CTA's column sums are with the others
+  if (grp == 1 && !has_mean) quant_v(nullptr);
+  cluster_wait();
+  if (has_mean) {
+    if (gt < HD) {
+      const double* part = reinterpret_cast<const double*>(gbase + L::PART) + grp * SHORT_CTAS * HD;
+      double t = 0.0;
+      for (uint32_t r = 0; r < C; ++r) t += part[r * HD + gt];
+      const float m = (float)(t / (double)a.N);
+      mean_s[gt] = m;
+      if (rank == 0) (grp == 0 ? sa.mean : sa.vmean)[(size_t)bh * HD + gt] = m;
+    }
+    half_sync();
+  }
+  if (grp == 0) {
+    landed();
+    quant_k_tile<T, INT8>(a, stage, mean_s, bh, n_base, a.N, c, r0);
+  } else {
+    if (has_mean) quant_v(mean_s);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) svmax = fmaxf(svmax, __shfl_xor_sync(0xffffffffu, svmax, off));
+    if (lane < (int)C)               // non-negative floats order like their bits
+      asm volatile("red.relaxed.cluster.shared::cluster.max.u32 [%0], %1;"
+                   ::"r"(in_cta(base + L::SVMAX, (uint32_t)lane)), "r"(__float_as_uint(svmax)) : "memory");
+  }
+  cluster_arrive();
+  cluster_wait();                    // the head's largest V scale is complete
+  if (grp == 1) {
+    const float S = fmaxf(__uint_as_float(*svmax_s), 1.0f);
+    if (rank == 0 && gt == 0) a.s_fold[bh] = S;
+    if (gt < TILE) a.svp[(size_t)bh * a.N_pad + n_base + gt] = __fmul_rn(__fdiv_rn(sv_s[gt], S), F8_MAX);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
 // Host launcher.
 // ------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -663,6 +874,35 @@ static bool make_map4(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, i
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <typename T, bool INT8>
+static cudaError_t launch_short(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const QuantArgs& a,
+                                const ShortArgs& sa, int64_t tiles_k, cudaStream_t st) {
+  auto kern = quant_short_kernel<T, INT8>;
+  static bool opted_in[64] = {false};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64 || !opted_in[dev]) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)short_smem::BYTES);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) opted_in[dev] = true;
+  }
+  const unsigned ctas = (unsigned)tiles_k;                              // per cluster
+  const int64_t per_cluster = (int64_t)ctas * 2;                        // Q tiles a cluster takes
+  const unsigned clusters = (unsigned)(sa.kv_clusters + (sa.items_q + per_cluster - 1) / per_cluster);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(clusters * ctas); cfg.blockDim = dim3(512); cfg.dynamicSmemBytes = short_smem::BYTES; cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = ctas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, a, sa);
+}
+
 template <typename T>
 static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
   const int64_t bh = p.B * p.H;
@@ -679,41 +919,6 @@ static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
     e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
   }
-  if (p.plan)
-    e = launch_after_predecessor(plan_packed_kernel, dim3(1), dim3(PLAN_MAX_SEQS), 0, st, words, (int)CtrlHeader::words(bh),
-                                 p.plan, (int)p.B, p.cu_q, p.cu_k, (long long)p.Tq, (long long)p.Tk, (long long)p.Nq,
-                                 (long long)p.N);
-  else
-    e = launch_after_predecessor(clear_ctrl_kernel, dim3(1), dim3(256), 0, st, words, (int)CtrlHeader::words(bh));
-  if (e != cudaSuccess) return e;
-  int nsplit = std::min(kmean_splits(bh, p.N, sm_count[dev]), kmean_splits_max(bh, p.N));
-  // A packed batch: chunks of 1 024 tokens whatever the number of heads, since its longest sequence
-  // would otherwise keep single CTAs busy long after the others (36 k tokens x 48 heads in eleven
-  // sequences of up to 8 192: 262 us with one CTA per sequence and head).  CTAs past a sequence's end leave.
-  if (p.partial && p.cu_k) {
-    const int64_t want = std::min<int64_t>((p.N + 1023) / 1024, (int64_t)(p.partial_bytes / ((size_t)bh * HD * sizeof(double))));
-    if (want > nsplit) { nsplit = (int)std::min<int64_t>(want, 65535); partial = reinterpret_cast<double*>(p.partial); }
-  }
-  if (p.smooth_k) {
-    long long chunk = (p.N + nsplit - 1) / nsplit;
-    chunk = (chunk + 15) / 16 * 16;
-    dim3 grid(nsplit, (unsigned)bh);
-    auto kmean = p.cu_k ? kmean_kernel<T, true> : kmean_kernel<T, false>;
-    e = launch_after_predecessor(kmean, grid, dim3(256), 0, st, reinterpret_cast<const T*>(p.k), p.mean, partial, words,
-                                 (long long)p.N, (long long)p.H, (long long)p.k_strides[0], (long long)p.k_strides[1],
-                                 (long long)p.k_strides[2], nsplit, chunk, (int)p.D, p.cu_k, (long long)p.Tk);
-    if (e != cudaSuccess) return e;
-  }
-  if (p.vmean) {
-    long long chunk = (p.N + nsplit - 1) / nsplit;
-    chunk = (chunk + 15) / 16 * 16;
-    dim3 grid(nsplit, (unsigned)bh);
-    auto kmean = p.cu_k ? kmean_kernel<T, true> : kmean_kernel<T, false>;
-    e = launch_after_predecessor(kmean, grid, dim3(256), 0, st, reinterpret_cast<const T*>(p.v), p.vmean, partial, words + 3 * bh,
-                                 (long long)p.N, (long long)p.H, (long long)p.v_strides[0], (long long)p.v_strides[1],
-                                 (long long)p.v_strides[2], nsplit, chunk, (int)p.D, p.cu_k, (long long)p.Tk);
-    if (e != cudaSuccess) return e;
-  }
   QuantArgs a;
   a.q8 = reinterpret_cast<uint8_t*>(p.q8); a.k8 = reinterpret_cast<uint8_t*>(p.k8);
   a.v8t = reinterpret_cast<uint8_t*>(p.v8t);
@@ -723,7 +928,7 @@ static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
   a.Nq = p.Nq; a.Hq = p.Hq; a.group = p.Hq / p.H; a.BHq = p.B * p.Hq; a.BHkv = bh; a.qm = p.qm;
   a.sub_mean = p.smooth_k ? 1 : 0;
   a.cu_q = p.cu_q; a.cu_k = p.cu_k; a.Tq = p.Tq; a.Tk = p.Tk;
-  a.plan = p.plan; a.n_seq = (int)p.B;
+  a.plan = p.plan; a.n_seq = (int)p.B; a.only_q = 0; a.drawn = 0;
   const bool varlen = p.cu_q != nullptr;
   const int64_t tq = (p.Nq + TILE - 1) / TILE, tk = p.N_pad / TILE;
   a.status = reinterpret_cast<int32_t*>(words + CtrlHeader::status_word(bh));
@@ -744,7 +949,60 @@ static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
              !make_map4(&mk, p.k, dt, p.D, p.N, p.H, p.B, p.k_strides) ||
              !make_map4(&mv, p.v, dt, p.D, p.N, p.H, p.B, p.v_strides))
     return cudaErrorInvalidValue;
-  const long long total = 2 * (long long)bh * tk + (long long)a.BHq * tq;
+  // Short calls take one launch, see quant_short_kernel.  Its CTAs do one tile each and wait for
+  // each other, so that it pays while there are at most about two and a half rounds of them (two to
+  // an SM); longer calls are bound by bandwidth, which the persistent quantiser uses better.  Whole
+  // call, with the short form / without, us: 48 heads of 288 tokens 19.8 / 25.3 (288 CTAs), 1 024
+  // tokens 58.2 / 62.3 (576), 1 100 tokens 63.3 / 69.1 (648), 1 536 tokens 100 / 95 (864), 2 048
+  // tokens 169 / 154 (1 152); 8 heads of 2 048 tokens 50.4 / 56.4 (192); 40 heads, 8 192 queries of
+  // 1 024 keys 236 / 231 (1 600).
+  if (!varlen && tk <= SHORT_CTAS && bh * tk + (a.BHq * tq + 1) / 2 <= 5 * (int64_t)sm_count[dev]) {
+    ShortArgs sa;
+    sa.mean = p.mean; sa.vmean = p.vmean; sa.words = words; sa.n_words = (int)CtrlHeader::words(bh); sa.kv_clusters = (int)bh;
+    sa.items_q = a.qm ? 0 : a.BHq * tq;      // Q tiles that need K's mean (for the LSE) follow in a launch of their own
+    sa.counter_word = (int)CtrlHeader::status_word(bh) + 2;
+    sa.items = (unsigned)(2 * bh * tk + sa.items_q);
+    e = (p.qk_mode == 0) ? launch_short<T, true>(mq, mk, mv, a, sa, tk, st) : launch_short<T, false>(mq, mk, mv, a, sa, tk, st);
+    if (e != cudaSuccess || sa.items_q > 0) return e;
+    a.only_q = 1; a.drawn = sa.items;
+  } else {
+    if (p.plan)
+      e = launch_after_predecessor(plan_packed_kernel, dim3(1), dim3(PLAN_MAX_SEQS), 0, st, words, (int)CtrlHeader::words(bh),
+                                   p.plan, (int)p.B, p.cu_q, p.cu_k, (long long)p.Tq, (long long)p.Tk, (long long)p.Nq,
+                                   (long long)p.N);
+    else
+      e = launch_after_predecessor(clear_ctrl_kernel, dim3(1), dim3(256), 0, st, words, (int)CtrlHeader::words(bh));
+    if (e != cudaSuccess) return e;
+    int nsplit = std::min(kmean_splits(bh, p.N, sm_count[dev]), kmean_splits_max(bh, p.N));
+    // A packed batch: chunks of 1 024 tokens whatever the number of heads, since its longest sequence
+    // would otherwise keep single CTAs busy long after the others (36 k tokens x 48 heads in eleven
+    // sequences of up to 8 192: 262 us with one CTA per sequence and head).  CTAs past a sequence's end leave.
+    if (p.partial && p.cu_k) {
+      const int64_t want = std::min<int64_t>((p.N + 1023) / 1024, (int64_t)(p.partial_bytes / ((size_t)bh * HD * sizeof(double))));
+      if (want > nsplit) { nsplit = (int)std::min<int64_t>(want, 65535); partial = reinterpret_cast<double*>(p.partial); }
+    }
+    if (p.smooth_k) {
+      long long chunk = (p.N + nsplit - 1) / nsplit;
+      chunk = (chunk + 15) / 16 * 16;
+      dim3 grid(nsplit, (unsigned)bh);
+      auto kmean = p.cu_k ? kmean_kernel<T, true> : kmean_kernel<T, false>;
+      e = launch_after_predecessor(kmean, grid, dim3(256), 0, st, reinterpret_cast<const T*>(p.k), p.mean, partial, words,
+                                   (long long)p.N, (long long)p.H, (long long)p.k_strides[0], (long long)p.k_strides[1],
+                                   (long long)p.k_strides[2], nsplit, chunk, (int)p.D, p.cu_k, (long long)p.Tk);
+      if (e != cudaSuccess) return e;
+    }
+    if (p.vmean) {
+      long long chunk = (p.N + nsplit - 1) / nsplit;
+      chunk = (chunk + 15) / 16 * 16;
+      dim3 grid(nsplit, (unsigned)bh);
+      auto kmean = p.cu_k ? kmean_kernel<T, true> : kmean_kernel<T, false>;
+      e = launch_after_predecessor(kmean, grid, dim3(256), 0, st, reinterpret_cast<const T*>(p.v), p.vmean, partial, words + 3 * bh,
+                                   (long long)p.N, (long long)p.H, (long long)p.v_strides[0], (long long)p.v_strides[1],
+                                   (long long)p.v_strides[2], nsplit, chunk, (int)p.D, p.cu_k, (long long)p.Tk);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  const long long total = (a.only_q ? 0 : 2 * (long long)bh * tk) + (long long)a.BHq * tq;
   long long ctas = (long long)sm_count[dev] * QT_MINBLOCKS;
   if (ctas > total) ctas = total;
   auto kern = varlen ? ((p.qk_mode == 0) ? quant_qkv_kernel<T, true, true> : quant_qkv_kernel<T, false, true>)
