@@ -282,6 +282,21 @@ __device__ __forceinline__ uint64_t kmajor_nosw_desc(uint32_t saddr) {
 constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr uint32_t IDESC_F8 = (1u << 4) | (0u << 7) | (0u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
+// w[k] of lane c (of four neighbouring lanes) becomes w[c] of lane k.
+__device__ __forceinline__ void transpose4(uint32_t (&w)[4], int c) {
+  const bool odd = c & 1, high = c & 2;
+#pragma unroll
+  for (int k = 0; k < 4; k += 2) {
+    const uint32_t r = __shfl_xor_sync(0xffffffffu, odd ? w[k] : w[k + 1], 1);
+    if (odd) w[k] = r; else w[k + 1] = r;
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t r = __shfl_xor_sync(0xffffffffu, high ? w[k] : w[k + 2], 2);
+    if (high) w[k] = r; else w[k + 2] = r;
+  }
+}
+
 struct AttnKArgs {
   const float *sq, *sk, *svp, *s_fold;
   void* out;
@@ -981,10 +996,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             a.lse[(size_t)bh * a.Nq + q_rowB] = v;
           }
         }
-        OutT* orowA = reinterpret_cast<OutT*>(a.out) + (VARLEN ? o_first : b * a.o_sb) + h * a.o_sh + q_rowA * a.o_sr + 2 * c;
+        OutT* orowA = reinterpret_cast<OutT*>(a.out) + (VARLEN ? o_first : b * a.o_sb) + h * a.o_sh + q_rowA * a.o_sr + 8 * c;
         OutT* orowB = orowA + 8 * a.o_sr;
         if (ROWS == RAGGED && a.heads_per_unit > 1) {   // rows of a folded unit: heads_per_unit heads of rows_per_head rows
-          const long long o_unit = b * a.o_sb + h * a.heads_per_unit * a.o_sh + 2 * c;
+          const long long o_unit = b * a.o_sb + h * a.heads_per_unit * a.o_sh + 8 * c;
           const unsigned hA = (unsigned)q_rowA / (unsigned)a.rows_per_head, hB = (unsigned)q_rowB / (unsigned)a.rows_per_head;
           orowA = reinterpret_cast<OutT*>(a.out) + o_unit + hA * a.o_sh + (q_rowA - (long long)hA * a.rows_per_head) * a.o_sr;
           orowB = reinterpret_cast<OutT*>(a.out) + o_unit + hB * a.o_sh + (q_rowB - (long long)hB * a.rows_per_head) * a.o_sr;
@@ -993,17 +1008,30 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         uint32_t o[64];
         tmem_ld_16x256b_x16(t_o, o);
         tmem_ld_wait();
+        // A thread holds channels 8i + 2c, 8i + 2c + 1.  The four threads of a row exchange words, so
+        // that each writes whole 16-byte blocks and a warp's store covers 64 contiguous bytes of a
+        // row instead of 16 (32 stores of 4 bytes became 8 of 16): 40 heads, 16 384 queries of
+        // 512 keys 235 -> 218 us, 48 x 2 048 x 2 048 113 -> 108, 48 x 8 771 x 8 771 1 596 -> 1 558.
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {                      // channels 8i + 2c, 8i + 2c + 1
-          if (8 * i + 2 * c < a.D) {
+        for (int i4 = 0; i4 < 4; ++i4) {
+          uint32_t wa[4], wb[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int i = 4 * i4 + k;
             float fa0 = __uint_as_float(o[4 * i + 0]) * invA, fa1 = __uint_as_float(o[4 * i + 1]) * invA;
             float fb0 = __uint_as_float(o[4 * i + 2]) * invB, fb1 = __uint_as_float(o[4 * i + 3]) * invB;
             if (vm != nullptr) {                            // smooth_v: the rows of P sum to one, so add the mean back
               const float2 mu = __ldg(reinterpret_cast<const float2*>(vm + 8 * i));
               fa0 += mu.x; fa1 += mu.y; fb0 += mu.x; fb1 += mu.y;
             }
-            if (q_rowA < (VARLEN ? Nq_live : a.Nq)) *reinterpret_cast<uint32_t*>(orowA + 8 * i) = pack2<OutT>(fa0, fa1);
-            if (q_rowB < (VARLEN ? Nq_live : a.Nq)) *reinterpret_cast<uint32_t*>(orowB + 8 * i) = pack2<OutT>(fb0, fb1);
+            wa[k] = pack2<OutT>(fa0, fa1);
+            wb[k] = pack2<OutT>(fb0, fb1);
+          }
+          transpose4(wa, c);
+          transpose4(wb, c);
+          if (32 * i4 + 8 * c < a.D) {
+            if (q_rowA < (VARLEN ? Nq_live : a.Nq)) *reinterpret_cast<uint4*>(orowA + 32 * i4) = make_uint4(wa[0], wa[1], wa[2], wa[3]);
+            if (q_rowB < (VARLEN ? Nq_live : a.Nq)) *reinterpret_cast<uint4*>(orowB + 32 * i4) = make_uint4(wb[0], wb[1], wb[2], wb[3]);
           }
         }
         }
