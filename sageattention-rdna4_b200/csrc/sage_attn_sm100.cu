@@ -445,6 +445,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     misc[1] = (*reinterpret_cast<volatile int32_t*>(a.status) != 0) ? 1u : 0u;
     if (FAST) { misc[4] = 0u; misc[5] = 0u; misc[6] = 0u; misc[7] = 0u; }   // skipped-warp counts, see the MMA issuer
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (NQ == 1) {                                          // the first loads do not wait for the rest of the CTA
+      mbar_expect_tx(bar(BAR_Q), TILE_BYTES);
+      tma_load_3d(base + OFF_Q, &tm_q, bar(BAR_Q), 0, q_tile0 * TILE, bh);
+      mbar_expect_tx(bar(BAR_KF), TILE_BYTES + 2 * VEC_BYTES);
+      tma_load_3d(base + OFF_K, &tm_k, bar(BAR_KF), 0, k_tile0 * TILE, bh_kv);
+      bulk_load(base + OFF_SK, a.sk + (size_t)bh_kv * a.N_pad + (size_t)k_tile0 * TILE, VEC_BYTES, bar(BAR_KF));
+      bulk_load(base + OFF_SV, a.svp + (size_t)bh_kv * a.N_pad + (size_t)k_tile0 * TILE, VEC_BYTES, bar(BAR_KF));
+    }
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -560,10 +568,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     } else if (warp == 0) {
       // ------------------------------- TMA producer (one query tile per CTA) ------
       if (lane == 0) {
-        prefetch_map(&tm_q); prefetch_map(&tm_k); prefetch_map(&tm_v);
-        mbar_expect_tx(bar(BAR_Q), NQ * TILE_BYTES);
-        for (int g = 0; g < NQ; ++g)                          // rows past the last query arrive as zeros
-          tma_load_3d(base + OFF_Q + g * TILE_BYTES, &tm_q, bar(BAR_Q), 0, (q_tile0 + g) * TILE, bh);
         const float* sk_row = a.sk + (size_t)bh_kv * a.N_pad + (size_t)k_tile0 * TILE;
         const float* sv_row = a.svp + (size_t)bh_kv * a.N_pad + (size_t)k_tile0 * TILE;
         auto load_k = [&](int j) -> bool {
@@ -579,7 +583,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           return true;
         };
         bool ok = true;
-        for (int j = 0; ok && j < L::K_AHEAD && j < n_load; ++j) ok = load_k(j);
+        // (Q and the first K tile are on their way, K_AHEAD is 1)
         for (int j = 0; ok && j < n_load; ++j) {
           if (j + L::K_AHEAD < n_load && !load_k(j + L::K_AHEAD)) break;
           if (ROWS == SPLIT_MAX) continue;                   // no P.V
