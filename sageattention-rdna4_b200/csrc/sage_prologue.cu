@@ -187,13 +187,6 @@ struct QuantArgs {
   long long drawn;                // items the work counter starts from: those that are done
 };
 
-// rn(x / s) given rc = rn(1/s)
-__device__ __forceinline__ float div_by_scale(float x, float s, float rc) {
-  const float q0 = __fmul_rn(x, rc);
-  const float r = -__fmaf_rn(q0, s, -x);      // x - q0*s, written so that a zero keeps x's sign
-  return __fmaf_rn(r, rc, q0);
-}
-
 // ------------------------------------------------------------------------------------------------
 // Kernel 2: persistent CTAs (three per SM) draw 128-token tiles of K, V and Q from one global work
 // counter; thread 0 keeps the next tile's 32 KB tensor-map load in flight into a shared-memory
@@ -202,6 +195,10 @@ __device__ __forceinline__ float div_by_scale(float x, float s, float rc) {
 // Thread (c = tid & 7, r0 = tid >> 3) owns columns 8c..8c+7 and 64+8c..64+8c+7 of rows r0, r0+32,
 // r0+64, r0+96: a quarter-warp reads one 256-byte row with two conflict-free 16-byte loads and the
 // row maximum is three shuffles.
+// Bound by HBM for long calls (48 heads x 47 520 tokens: 489 us, 2.6 GB), by instructions between the
+// round trips otherwise: quotients for e4m3 two at a time, magnitudes on the packed 16-bit values,
+// items worked out by one thread and one barrier less per item took 48 x 4 096 from 53 to 48 us, 24 x
+// 27 280 (bf16) from 152 to 142 and 36 k packed tokens x 48 heads from 526 to 400.
 // ------------------------------------------------------------------------------------------------
 constexpr int QT_STAGES = 2;        // shared-memory ring: one tile being quantised, one in flight
 constexpr int QT_MINBLOCKS = 3;     // CTAs per SM (3 x 64 KB of shared memory, 80 registers per thread)
@@ -238,6 +235,35 @@ __device__ __forceinline__ uint32_t i8x4_magic2(float2 ab, float2 cd) {
                      __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x0040), 0x5410);
 }
 
+// Largest magnitude of eight packed 16-bit values: exact on the packed form, half the instructions.
+template <typename T> struct Packed16;
+template <> struct Packed16<__half> { typedef __half2 Pair; };
+template <> struct Packed16<__nv_bfloat16> { typedef __nv_bfloat162 Pair; };
+template <typename T>
+__device__ __forceinline__ float absmax16(const uint4& u, const uint4& v) {
+  typedef typename Packed16<T>::Pair Pair;
+  const uint32_t w[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+  Pair m = __habs2(*reinterpret_cast<const Pair*>(&w[0]));
+#pragma unroll
+  for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const Pair*>(&w[i])));
+  const float2 f = Elem<T>::cvt2(*reinterpret_cast<const uint32_t*>(&m));
+  return fmaxf(f.x, f.y);
+}
+__device__ __forceinline__ float absmax3(float m, float2 x) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(fabsf(x.x)), "f"(fabsf(x.y)));
+  return r;
+}
+// e4m3 codes of rn(x / s) for four values, given rc = rn(1/s).  The remainder is taken as q0*s - x and
+// subtracted, which keeps the sign of a zero x; the packed operations have no negation, so the
+// steps divide -x (all signs turn around, those of zeros too) and the codes' sign bits are flipped back.
+__device__ __forceinline__ uint32_t e4m3x4_quot(float2 a, float2 b, float s, float rc) {
+  const float2 nrc = make_float2(-rc, -rc), s2 = make_float2(s, s);
+  const float2 qa = __fmul2_rn(a, nrc), qb = __fmul2_rn(b, nrc);
+  const float2 ya = __ffma2_rn(__ffma2_rn(qa, s2, a), nrc, qa), yb = __ffma2_rn(__ffma2_rn(qb, s2, b), nrc, qb);
+  return e4m3x4(ya.x, ya.y, yb.x, yb.y) ^ 0x80808080u;
+}
+
 // ------------------------------------------------------------------------------------------------
 // One 128-token tile, already in shared memory (128 rows of 256 bytes), by 256 threads.  Thread
 // (c = tid & 7, r0 = tid >> 3) owns columns 8c..8c+7 and 64+8c..64+8c+7 of rows r0, r0+32, r0+64,
@@ -259,12 +285,10 @@ __device__ __forceinline__ void quant_q_tile(const QuantArgs& a, const uint8_t* 
     const int t = r0 + 32 * i;
     const long long nrow = n_base + t;
     float x[16];
-    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
-    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
-    float amax = 0.f;
-#pragma unroll
-    for (int e = 0; e < 16; ++e) amax = fmaxf(amax, fabsf(x[e]));
-    amax = fmaxf(quarter_warp_max(amax), SCALE_FLOOR);
+    const uint4 u0 = *reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), u1 = *reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c);
+    unpack8<T>(u0, x);
+    unpack8<T>(u1, x + 8);
+    const float amax = fmaxf(quarter_warp_max(absmax16<T>(u0, u1)), SCALE_FLOOR);
     const float qinv = __fdiv_rn(QMAX, amax);
     float2 y[8];
 #pragma unroll
@@ -321,7 +345,7 @@ __device__ __forceinline__ void quant_k_tile(const QuantArgs& a, const uint8_t* 
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       xs[e] = __fadd2_rn(make_float2(x[2 * e], x[2 * e + 1]), nmu[e]);
-      amax = fmaxf(amax, fmaxf(fabsf(xs[e].x), fabsf(xs[e].y)));
+      amax = absmax3(amax, xs[e]);
     }
     amax = quarter_warp_max(live ? amax : 0.f);
     const float sk = fmaxf(div_const<QDIV>(amax), SCALE_FLOOR);
@@ -340,11 +364,8 @@ __device__ __forceinline__ void quant_k_tile(const QuantArgs& a, const uint8_t* 
       w0.x = i8x4_magic2(y[0], y[1]); w0.y = i8x4_magic2(y[2], y[3]);
       w1.x = i8x4_magic2(y[4], y[5]); w1.y = i8x4_magic2(y[6], y[7]);
     } else {
-      float y[16];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { y[2 * e] = div_by_scale(xs[e].x, sk, rc); y[2 * e + 1] = div_by_scale(xs[e].y, sk, rc); }
-      w0.x = e4m3x4(y[0], y[1], y[2], y[3]); w0.y = e4m3x4(y[4], y[5], y[6], y[7]);
-      w1.x = e4m3x4(y[8], y[9], y[10], y[11]); w1.y = e4m3x4(y[12], y[13], y[14], y[15]);
+      w0.x = e4m3x4_quot(xs[0], xs[1], sk, rc); w0.y = e4m3x4_quot(xs[2], xs[3], sk, rc);
+      w1.x = e4m3x4_quot(xs[4], xs[5], sk, rc); w1.y = e4m3x4_quot(xs[6], xs[7], sk, rc);
     }
     if (!live) { w0 = make_uint2(0u, 0u); w1 = w0; }
     // rows are stored permuted inside 16-row blocks: key 4cc + jj of a block goes to row
@@ -368,12 +389,6 @@ __device__ __forceinline__ float quant_v_tile(const QuantArgs& a, uint8_t* st, c
                                               long long n_base, long long N, int tid) {
   const int c = tid & 7, r0 = tid >> 3, lane = tid & 31, warp = tid >> 5;
   const long long N_pad = a.N_pad;
-  float vmu[16];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    vmu[e] = vmean ? vmean[8 * c + e] : 0.f;
-    vmu[8 + e] = vmean ? vmean[64 + 8 * c + e] : 0.f;
-  }
   float svmax = 0.f;
   uint2 w0[4], w1[4];
 #pragma unroll
@@ -382,23 +397,31 @@ __device__ __forceinline__ float quant_v_tile(const QuantArgs& a, uint8_t* st, c
     const long long nrow = n_base + t;
     const bool live = nrow < N;
     float x[16];
-    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), x);
-    unpack8<T>(*reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c), x + 8);
-    float amax = 0.f;
+    const uint4 u0 = *reinterpret_cast<const uint4*>(st + t * 256 + 16 * c), u1 = *reinterpret_cast<const uint4*>(st + t * 256 + 128 + 16 * c);
+    unpack8<T>(u0, x);
+    unpack8<T>(u1, x + 8);
+    float amax;
+    if (vmean) {
+      amax = 0.f;
 #pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      if (vmean) x[e] = live ? __fsub_rn(x[e], vmu[e]) : 0.f;
-      if (VARLEN && !live) x[e] = 0.f;               // the rows behind a packed sequence are its neighbour's
-      amax = fmaxf(amax, fabsf(x[e]));
+      for (int e = 0; e < 16; ++e) {
+        x[e] = live ? __fsub_rn(x[e], vmean[(e < 8 ? 0 : 56) + 8 * c + e]) : 0.f;
+        amax = fmaxf(amax, fabsf(x[e]));
+      }
+    } else {
+      amax = absmax16<T>(u0, u1);
+      if (VARLEN && !live) {                               // the rows behind a packed sequence are its neighbour's
+        amax = 0.f;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) x[e] = 0.f;
+      }
     }
     amax = quarter_warp_max(amax);
     const float sv = fmaxf(div_const<448>(amax), SCALE_FLOOR);
     const float rc = __frcp_rn(sv);
-    float y[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e) y[e] = div_by_scale(x[e], sv, rc);
-    w0[i].x = e4m3x4(y[0], y[1], y[2], y[3]); w0[i].y = e4m3x4(y[4], y[5], y[6], y[7]);
-    w1[i].x = e4m3x4(y[8], y[9], y[10], y[11]); w1[i].y = e4m3x4(y[12], y[13], y[14], y[15]);
+    const float2* x2 = reinterpret_cast<const float2*>(x);
+    w0[i].x = e4m3x4_quot(x2[0], x2[1], sv, rc); w0[i].y = e4m3x4_quot(x2[2], x2[3], sv, rc);
+    w1[i].x = e4m3x4_quot(x2[4], x2[5], sv, rc); w1[i].y = e4m3x4_quot(x2[6], x2[7], sv, rc);
     if (c == 0) {
       a.sv[(size_t)bh * N_pad + nrow] = live ? sv : 0.0f;
       if (sv_tile) sv_tile[t] = live ? sv : 0.0f;
@@ -450,7 +473,7 @@ __global__ void __launch_bounds__(256, QT_MINBLOCKS)
 quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const QuantArgs a) {
   extern __shared__ uint8_t qt_smem[];
-  __shared__ long long s_item[QT_STAGES];
+  __shared__ int4 s_item[QT_STAGES];   // what the stage holds: {tensor (0 q, 1 k, 2 v, 3 a fold, -1 the end), head, tile, live tokens}
   __shared__ int s_plan[VARLEN ? 4 * (PLAN_MAX_SEQS + 1) : 1];
   const uint32_t raw_addr = qt_smem_u32(qt_smem);
   const uint32_t base = (raw_addr + 127u) & ~127u;
@@ -466,50 +489,51 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   wait_for_predecessor();            // the means and the cleared control block
   allow_successor();                 // persistent grid: every CTA is resident
 
-  const long long tiles_q = (a.Nq + TILE - 1) / TILE, tiles_k = a.N_pad / TILE;
-  const long long items_k = a.only_q ? 0 : a.BHkv * tiles_k, items_q = a.BHq * tiles_q;
-  const long long fold_per_head = (a.N_pad + FOLD_KEYS - 1) / FOLD_KEYS;
-  const long long items_f = a.only_q ? 0 : a.BHkv * fold_per_head;
   const bool planned = VARLEN && a.plan != nullptr;
   const int P1 = VARLEN ? a.n_seq + 1 : 0;
   if (planned) {
     for (int i = tid; i < 4 * P1; i += 256) s_plan[i] = a.plan[i];
     __syncthreads();
   }
-  const long long live_k = planned ? s_plan[3 * P1 - 1] * a.H : items_k, live_q = planned ? s_plan[2 * P1 - 1] * a.Hq : items_q;
-  const long long total = 2 * live_k + live_q + (planned ? s_plan[4 * P1 - 1] * a.H : items_f);
+  // Counts of items fit 32 bits: every K, V or Q item stands for 16 KB of codes.
+  const int tiles_q = (int)((a.Nq + TILE - 1) / TILE), tiles_k = (int)(a.N_pad / TILE);
+  const int fold_per_head = (int)((a.N_pad + FOLD_KEYS - 1) / FOLD_KEYS);
+  const int items_k = a.only_q ? 0 : planned ? s_plan[3 * P1 - 1] * (int)a.H : (int)a.BHkv * tiles_k;
+  const int items_q = planned ? s_plan[2 * P1 - 1] * (int)a.Hq : (int)a.BHq * tiles_q;
+  const int items_f = a.only_q ? 0 : planned ? s_plan[4 * P1 - 1] * (int)a.H : (int)a.BHkv * fold_per_head;
+  const int total = 2 * items_k + items_q + items_f;
 
   // item -> (tensor, head, tile): K first with the last heads first (their rows are still in L2
-  // after the mean pass), then V (so that the per-head folds overlap the Q items), then Q
-  auto decode = [&](long long it, int& which, long long& bh, long long& tile) {
-    if (planned) {                     // sequence by sequence in the plan's order, head by head
-      int arr = 2;
-      int j;
-      if (it < live_k) { which = 1; j = (int)it; }
-      else if (it < 2 * live_k) { which = 2; j = (int)(it - live_k); }
-      else if (it < 2 * live_k + live_q) { which = 0; j = (int)(it - 2 * live_k); arr = 1; }
-      else { which = 3; j = (int)(it - 2 * live_k - live_q); arr = 3; }
+  // after the mean pass), then V (so that the per-head folds overlap the Q items), then Q, then the
+  // folds.  With a work list: sequence by sequence in the list's order, head by head.
+  auto decode = [&](int it, int& which, int& bh, int& tile) {
+    int j = it;
+    if (it < items_k) which = 1;
+    else if (it < 2 * items_k) { which = 2; j -= items_k; }
+    else if (it < 2 * items_k + items_q) { which = 0; j -= 2 * items_k; }
+    else { which = 3; j -= 2 * items_k + items_q; }
+    if (planned) {
       const int heads = (int)((which == 0) ? a.Hq : a.H);
-      const int* pre = s_plan + arr * P1;
+      const int* pre = s_plan + (which == 0 ? 1 : which == 3 ? 3 : 2) * P1;
       int lo = 0, hi = a.n_seq;        // pre[lo] * heads <= j < pre[hi] * heads
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if ((long long)pre[mid] * heads <= j) lo = mid; else hi = mid;
+        if (pre[mid] * heads <= j) lo = mid; else hi = mid;
       }
       const int rem = j - pre[lo] * heads, per = pre[lo + 1] - pre[lo];
-      bh = (long long)s_plan[lo] * heads + rem / per;
+      bh = s_plan[lo] * heads + rem / per;
       tile = rem % per;
-      return;
+    } else {
+      const int per = (which == 0) ? tiles_q : which == 3 ? fold_per_head : tiles_k;
+      const int r = j / per;
+      bh = (int)((which == 0) ? a.BHq : a.BHkv) - 1 - r;
+      tile = j - r * per;
     }
-    if (it < items_k) { which = 1; bh = a.BHkv - 1 - it / tiles_k; tile = it % tiles_k; }
-    else if (it < 2 * items_k) { const long long j = it - items_k; which = 2; bh = a.BHkv - 1 - j / tiles_k; tile = j % tiles_k; }
-    else if (it < 2 * items_k + items_q) { const long long j = it - 2 * items_k; which = 0; bh = a.BHq - 1 - j / tiles_q; tile = j % tiles_q; }
-    else { const long long j = it - 2 * items_k - items_q; which = 3; bh = a.BHkv - 1 - j / fold_per_head; tile = j % fold_per_head; }
   };
   // length and first input token of the sequence an item belongs to
-  auto seq_of = [&](int which, long long bh, long long& start) -> long long {
+  auto seq_of = [&](int which, int bh, long long& start) -> long long {
     if (!VARLEN) { start = 0; return (which == 0) ? a.Nq : a.N; }
-    const long long b = bh / ((which == 0) ? a.Hq : a.H);
+    const int b = bh / (int)((which == 0) ? a.Hq : a.H);
     const int* cu = (which == 0) ? a.cu_q : a.cu_k;
     // clamped to the packed tensor: whatever the arrays hold, a sequence lies inside it
     const long long T = (which == 0) ? a.Tq : a.Tk;
@@ -518,37 +542,27 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     return min(max(s1 - s0, 0LL), (which == 0) ? a.Nq : a.N);
   };
   // Items are handed out through one global counter: a CTA that is held up (by a head's fold, say)
-  // simply takes fewer of them.  Thread 0 publishes the item of a stage in s_item and starts its
-  // load; past the end it publishes -1 and completes the stage's barrier by hand.  The counter is
+  // simply takes fewer of them.  Thread 0 draws an item, works out what it is, publishes that in
+  // s_item and starts the load; the other threads see it with the stage's barrier.  The counter is
   // drawn one item ahead, so the atomic's round trip is off the critical path.
-  auto draw = [&]() { return (long long)atomicAdd(a.next_item, 1ULL) - a.drawn; };
-  auto issue = [&](int stage, long long it) {
+  auto draw = [&]() { return (int)((long long)atomicAdd(a.next_item, 1ULL) - a.drawn); };
+  auto issue = [&](int stage, int it) {
     const uint32_t bar_ = bar0 + 8u * (uint32_t)stage;
-    if (it >= total) {
-      s_item[stage] = -1;
+    int which = -1, bh = 0, tile = 0;
+    long long start = 0, len = 0;
+    if (it < total) {
+      decode(it, which, bh, tile);
+      len = seq_of(which == 3 ? 1 : which, bh, start);
+    }
+    s_item[stage] = make_int4(which, bh, tile, (int)len);
+    // the end, folds and tiles past their sequence's end load nothing
+    if (which < 0 || which == 3 || (VARLEN && (long long)tile * TILE >= len)) {
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_) : "memory");
       return;
     }
-    s_item[stage] = it;
-    int which; long long bh, tile;
-    decode(it, which, bh, tile);
-    if (which == 3) {                  // fold items read no tile
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_) : "memory");
-      return;
-    }
-    const long long heads = (which == 0) ? a.Hq : a.H;
-    int b = (int)(bh / heads);
-    const int h = (int)(bh - (long long)b * heads);
-    long long row = tile * TILE;
-    if (VARLEN) {                      // a tile past the sequence's end is not loaded; the map has one batch entry
-      long long start;
-      if (row >= seq_of(which, bh, start)) {
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_) : "memory");
-        return;
-      }
-      row += start;
-      b = 0;
-    }
+    const int heads = (int)((which == 0) ? a.Hq : a.H);
+    const int b = VARLEN ? 0 : bh / heads, h = bh % heads;        // (a packed batch's map has one batch entry)
+    const long long row = start + (long long)tile * TILE;
     const CUtensorMap* map = (which == 0) ? &tm_q : (which == 1 ? &tm_k : &tm_v);
     const uint32_t bar = bar0 + 8u * (uint32_t)stage, dst = base + (uint32_t)stage * QT_STAGE_BYTES;
     // the stage was last touched by ordinary loads and stores (V tiles are staged back into it);
@@ -561,11 +575,12 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   };
 
   __syncthreads();
-  long long drawn = 0;
+  int drawn = 0;
   if (tid == 0) {
     for (int p = 0; p < QT_STAGES - 1; ++p) issue(p, draw());
     drawn = draw();
   }
+  __syncthreads();                     // s_item of the first stage, for a thread whose wait runs out too
 
   for (uint32_t n = 0;; ++n) {
     const int stage = (int)(n % QT_STAGES);
@@ -574,33 +589,25 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       issue((int)((n + QT_STAGES - 1) % QT_STAGES), drawn);
       drawn = draw();                  // consumed one iteration later
     }
-    // bounded wait for this item's tile
-    int ok = 1;
+    // bounded wait for this item's tile; a thread that gives up goes on to the barrier at the end of
+    // the item, where all leave together
+    int lost = 0;
     {
       const uint32_t bar = bar0 + 8u * (uint32_t)stage;
       if (!qt_try_wait(bar, parity)) {
         const long long t0 = clock64();
         uint32_t spins = 0;
         while (!qt_try_wait(bar, parity)) {
-          if ((++spins & 1023u) == 0u && clock64() - t0 > QT_WAIT_CYCLES) { ok = 0; break; }
+          if ((++spins & 1023u) == 0u && clock64() - t0 > QT_WAIT_CYCLES) { lost = 1; break; }
         }
       }
     }
-    if (!__syncthreads_and(ok)) {
-      if (tid == 0) { atomicOr(a.status, 1); if (a.status2) atomicOr(a.status2, 8); }
-      const long long t0 = clock64();
-      while (clock64() - t0 < 400000) { }     // give copies still in flight a moment to land
-      break;
-    }
-
-    const long long it = s_item[stage];
-    if (it < 0) break;                 // the list is exhausted (every thread reads the same value)
-    int which; long long bh, tile;
-    decode(it, which, bh, tile);
-    const long long n_base = tile * TILE;
+    const int4 item = s_item[stage];
+    const int which = item.x;
+    if (which < 0) break;              // the list is exhausted (every thread reads the same value)
+    const int bh = item.y, tile = item.z, seq_len = item.w;
+    const long long n_base = (long long)tile * TILE;
     const uint8_t* st = gbase + (size_t)stage * QT_STAGE_BYTES;
-    long long seq_start;
-    const long long seq_len = seq_of(which == 3 ? 1 : which, bh, seq_start);
     const bool beyond = VARLEN && which != 3 && n_base >= seq_len;   // nothing was loaded, nothing is written
 
     if (beyond) {
@@ -644,12 +651,12 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         break;
       }
       const long long N_pad = a.N_pad;
-      const long long n_fold = VARLEN ? (seq_len + TILE - 1) / TILE * TILE : N_pad;   // rows that were written
+      const long long n_fold = VARLEN ? ((long long)seq_len + TILE - 1) / TILE * TILE : N_pad;   // rows that were written
       const float S = fmaxf(__uint_as_float(__ldcg(&a.svmax_bits[bh])), 1.0f);
       if (tile == 0 && tid == 0) a.s_fold[bh] = S;
 #pragma unroll
       for (int i = 0; i < FOLD_KEYS / 1024; ++i) {
-        const long long nn = tile * FOLD_KEYS + (long long)i * 1024 + 4 * tid;
+        const long long nn = (long long)tile * FOLD_KEYS + i * 1024 + 4 * tid;
         if (nn < n_fold) {             // a multiple of 128: whole float4s
           const float4 v = __ldcg(reinterpret_cast<const float4*>(a.sv + (size_t)bh * N_pad + nn));
           float4 o;
@@ -659,7 +666,12 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       }
     }
-    __syncthreads();                   // the stage may be refilled
+    if (__syncthreads_or(lost)) {      // the stage may be refilled
+      if (tid == 0) { atomicOr(a.status, 1); if (a.status2) atomicOr(a.status2, 8); }
+      const long long t0 = clock64();
+      while (clock64() - t0 < 400000) { }     // give copies still in flight a moment to land
+      break;
+    }
     if (which == 2 && !beyond && tid == 0) {   // this tile's V scales and maximum are published: one release per CTA
       __threadfence();
       atomicAdd(a.arrivals + bh, 1u);
