@@ -103,10 +103,10 @@ template <int NQ> struct Shape {
   __host__ __device__ static constexpr uint32_t tmem_o(int g) { return 128u * NQ + 128u * (uint32_t)g; }
 };
 
-// The K/V stage barriers are shared by the query tiles of a CTA; the last four repeat per query
+// The K/V stage barriers are shared by the query tiles of a CTA; the last six repeat per query
 // tile (+ BAR_PER_TILE x g).
 enum Bar { BAR_Q = 0, BAR_KF = 1, BAR_KE = 3, BAR_VF = 5, BAR_VE = 7, BAR_SF = 9, BAR_SFREE = 10,
-           BAR_PF = 11, BAR_PV = 12, BAR_PER_TILE = 4, BAR_COUNT = 17 };
+           BAR_PF = 11, BAR_PV = 13, BAR_PER_TILE = 6, BAR_COUNT = 21 };
 static_assert(BAR_COUNT * 8 <= 192, "barrier area");
 
 enum { ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_SOFTMAX = 4 };
@@ -439,8 +439,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (int g = 0; g < NQ; ++g) {
       mbar_init(bar(BAR_SF + BAR_PER_TILE * g), 1);
       mbar_init(bar(BAR_SFREE + BAR_PER_TILE * g), (uint32_t)live_warps(g));
-      mbar_init(bar(BAR_PF + BAR_PER_TILE * g), (uint32_t)live_warps(g));
-      mbar_init(bar(BAR_PV + BAR_PER_TILE * g), 1);
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(bar(BAR_PF + i + BAR_PER_TILE * g), (uint32_t)live_warps(g));
+        mbar_init(bar(BAR_PV + i + BAR_PER_TILE * g), 1);
+      }
     }
     misc[1] = (*reinterpret_cast<volatile int32_t*>(a.status) != 0) ? 1u : 0u;
     if (FAST) { misc[4] = 0u; misc[5] = 0u; misc[6] = 0u; misc[7] = 0u; }   // skipped-warp counts, see the MMA issuer
@@ -471,6 +473,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // never add up to more than the launch allocation.
   static_assert(128 * L::REGS_PRODUCER + 256 * NQ * L::REGS_SOFTMAX <= L::THREADS * L::REGS_AT_LAUNCH,
                 "setmaxnreg.inc would wait for registers that never become free");
+  // P.V(j-1): waited for on every key tile, or (PAIRED) only before the accumulator is rescaled.  The
+  // wait also keeps a softmax warp from overwriting P(j-2) while P.V(j-2) reads it and from getting two
+  // phases ahead of a barrier.  PAIRED puts that on S(j) instead: the Q.K^T issuer issues S(j) when
+  // P.V(j-2) is complete, and the P and P.V barriers exist once per P tile, so that the phase a
+  // thread looks for is never more than one behind.  In the two-tile shape that wait delays S, which pays
+  // where tiles are skipped (16 heads x 16 384 keys, 0.1 % dominant: 1 718 -> 1 634 us) and not where they
+  // are not (1 719 -> 1 762, 24 heads x 27 280: 6 884 -> 7 213); one issuing thread has its products
+  // in order anyway (48 x 4 096: 385 -> 382).
+  constexpr bool PAIRED = FAST || NQ == 1;
+  auto of_pair = [&](int first, int gb, int j) { return bar(first + gb + (PAIRED ? (j & 1) : 0)); };
+  auto pair_parity = [&](int j) { return (uint32_t)(PAIRED ? j >> 1 : j) & 1u; };
   if (!skip_all) {
     if (warp < 4) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::REGS_PRODUCER));
@@ -515,6 +528,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int j = 0; ok && j < n_tiles; ++j) {
             const int s = j & 1;
             ok = mbar_wait(bar(BAR_KF + s), (uint32_t)(j >> 1) & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
+            if (PAIRED && ok && j > 1) ok = mbar_wait(of_pair(BAR_PV, gb, j - 2), pair_parity(j - 2), cta_abort, a.status, ST_TIMEOUT_MMA);
             if (ok && j > 0) ok = mbar_wait(bar(BAR_SFREE + gb), (uint32_t)(j - 1) & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
             if (!ok) break;
             tc_fence_after();
@@ -542,7 +556,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int jj = 0; ok && jj < n_tiles; ++jj) {
             const int s = jj % L::V_STAGES;
             ok = mbar_wait(bar(BAR_VF + s), (uint32_t)(jj / L::V_STAGES) & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
-            if (ok) ok = mbar_wait(bar(BAR_PF + gb), (uint32_t)jj & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
+            if (ok) ok = mbar_wait(of_pair(BAR_PF, gb, jj), pair_parity(jj), cta_abort, a.status, ST_TIMEOUT_MMA);
             if (!ok) break;
             bool all_zero = false;
             if (FAST) {
@@ -560,7 +574,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                             kmajor_sw128_desc(base + OFF_V + s * TILE_BYTES + 32 * k), IDESC_F8,
                             (jj > 0 || k > 0) ? 1u : 0u);
             tc_commit(bar(BAR_VE + s));
-            tc_commit(bar(BAR_PV + gb));
+            tc_commit(of_pair(BAR_PV, gb, jj));
             if (warp == 3 && jj + L::V_STAGES < n_load) ok = load_v(jj + L::V_STAGES);
           }
         }
@@ -620,7 +634,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           if (ROWS != SPLIT_MAX && j > 0) {
             const int jj = j - 1, s = jj % L::V_STAGES;
             ok = mbar_wait(bar(BAR_VF + s), (uint32_t)(jj / L::V_STAGES) & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
-            if (ok) ok = mbar_wait(bar(BAR_PF + gb), (uint32_t)jj & 1u, cta_abort, a.status, ST_TIMEOUT_MMA);
+            if (ok) ok = mbar_wait(of_pair(BAR_PF, gb, jj), pair_parity(jj), cta_abort, a.status, ST_TIMEOUT_MMA);
             if (!ok) break;
             // FAST kernels: a warp that skips a tile counts itself before it arrives at the P
             // barrier.  When all live warps of the query tile did, P(jj) is all zeros and the
@@ -642,7 +656,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                             kmajor_sw128_desc(base + OFF_V + s * TILE_BYTES + 32 * k), IDESC_F8,
                             (jj > 0 || k > 0) ? 1u : 0u);
             tc_commit(bar(BAR_VE + s));
-            tc_commit(bar(BAR_PV + gb));
+            tc_commit(of_pair(BAR_PV, gb, jj));
           }
         }
       }
@@ -707,8 +721,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       constexpr uint32_t TRY_BOUND = 256u, ARMED = 512u, FAIL_ONE = 1u << 12, FAIL_MASK = 15u << 12;
       int n_skipped = 0;                                    // tiles this warp skipped (reported once, at the end)
       // What is left of a skipped tile: zeros for the warp's P rows (unless the tile already holds
-      // them), the wait for P.V(j-1) (see the comment at the other copy of this wait below) and
-      // the arrival at the P barrier.
+      // them) and the arrival at the P barrier.
       auto finish_skipped = [&](int j) -> bool {
         const uint32_t bit = 1u << (j & (L::P_BUFS - 1));
         if (!(fast & bit)) {
@@ -718,17 +731,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         fast = (fast & ~FAIL_MASK) | bit | TRY_BOUND | ARMED;
         ++n_skipped;
-        if (j > 0) {
-          const bool w = mbar_wait(bar(BAR_PV + gb), (uint32_t)(j - 1) & 1u, cta_abort, a.status, ST_TIMEOUT_SOFTMAX);
-          if (!__all_sync(0xffffffffu, w)) return false;
-          tc_fence_after();
-        }
-        // (after the wait: P.V(j-1) complete means the MMA thread has read and cleared the count of tile j-2)
+        // (S(j) complete means P.V(j-2) was issued: the issuer has read and cleared the count of tile j-2)
         if (lane == 0) atomicAdd(const_cast<uint32_t*>(misc) + 4 + 2 * g + (j & 1), 1u);
         fence_async_smem();
         tc_fence_before();
         __syncwarp();
-        mbar_arrive_lane0(bar(BAR_PF + gb), lane);
+        mbar_arrive_lane0(of_pair(BAR_PF, gb, j), lane);
         return true;
       };
 
@@ -917,13 +925,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         lB = lB * alphaB + (psB.x + psB.y);
         if (FAST) fast &= ~(1u << (j & (L::P_BUFS - 1)));
         // P.V(j-1) must be complete before the accumulator is rescaled.  The wait sits behind the
-        // exponentials, where it does not stall: P(j) went to the tile that P.V(j-2) read, and that
-        // product was waited for in the previous iteration.  It is made on every tile, rescaling
-        // or not: it also keeps this warp from arriving at the P barrier of tile j before the MMA
-        // thread has seen the barrier of tile j-1 complete (P.V(j-1) is issued after that), and
+        // exponentials, where it does not stall: P(j) went to the tile that P.V(j-2) read.  Unless
+        // PAIRED it is made on every tile, rescaling or not: it also keeps this warp from arriving at
+        // the P barrier of tile j before the MMA thread has seen the barrier of tile j-1 complete, and
         // the MMA thread's parity wait cannot tell a barrier that is two phases ahead.
-        if (j > 0) {
-          ok = mbar_wait(bar(BAR_PV + gb), (uint32_t)(j - 1) & 1u, cta_abort, a.status, ST_TIMEOUT_SOFTMAX);
+        if (PAIRED ? rescale : j > 0) {
+          ok = mbar_wait(of_pair(BAR_PV, gb, j - 1), pair_parity(j - 1), cta_abort, a.status, ST_TIMEOUT_SOFTMAX);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
@@ -946,7 +953,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         fence_async_smem();
         tc_fence_before();
         __syncwarp();
-        mbar_arrive_lane0(bar(BAR_PF + gb), lane);
+        mbar_arrive_lane0(of_pair(BAR_PF, gb, j), lane);
       }
 
       if (FAST && a.skipped != nullptr && lane == 0 && n_skipped > 0) atomicAdd(a.skipped, (unsigned)n_skipped);
@@ -959,7 +966,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         ok = false;
       }
       if (ok) {
-        ok = mbar_wait(bar(BAR_PV + gb), (uint32_t)(n_tiles - 1) & 1u, cta_abort, a.status, ST_TIMEOUT_SOFTMAX);
+        ok = mbar_wait(of_pair(BAR_PV, gb, n_tiles - 1), pair_parity(n_tiles - 1), cta_abort, a.status, ST_TIMEOUT_SOFTMAX);
         ok = __all_sync(0xffffffffu, ok);
       }
       if (ok) {
