@@ -97,12 +97,25 @@ plan_packed_kernel(unsigned* __restrict__ words, int n, int* __restrict__ plan, 
 // Kernel 1: partial fp64 column sums of K; the last CTA of a head combines them in split order.
 // grid (nsplit, B*H), block 256 = 16 row lanes x 16 column chunks of 8 elements.
 // ------------------------------------------------------------------------------------------------
+template <typename T> struct MeanOf {   // one tensor: its rows, where its mean, partial sums and arrival counters are
+  const T* x;
+  float* mean;
+  double* partial;
+  unsigned* arrivals;
+  long long sb, sh, sr;
+};
+// With smooth_v the means of K and V are one launch (blockIdx.z): each alone is mostly latency in
+// calls of this size (4 x 16 heads, 2 048 x 64: two launches of 13 us).
 template <typename T, bool VARLEN>
 __global__ void __launch_bounds__(256)
-kmean_kernel(const T* __restrict__ K, float* __restrict__ mean, double* __restrict__ partial,
-             unsigned* __restrict__ arrivals, long long N, long long H,
-             long long sb, long long sh, long long sr, int nsplit, long long chunk, int D,
+kmean_kernel(const MeanOf<T> of_k, const MeanOf<T> of_v, long long N, long long H, int nsplit, long long chunk, int D,
              const int* __restrict__ cu, long long tokens) {
+  const MeanOf<T>& of = (blockIdx.z == 0) ? of_k : of_v;
+  const T* __restrict__ K = of.x;
+  float* __restrict__ mean = of.mean;
+  double* __restrict__ partial = of.partial;
+  unsigned* __restrict__ arrivals = of.arrivals;
+  const long long sb = of.sb, sh = of.sh, sr = of.sr;
   __shared__ double red[16][HD];
   __shared__ int s_last;
   wait_for_predecessor();            // the cleared arrival counters
@@ -993,26 +1006,24 @@ static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
       const int64_t want = std::min<int64_t>((p.N + 1023) / 1024, (int64_t)(p.partial_bytes / ((size_t)bh * HD * sizeof(double))));
       if (want > nsplit) { nsplit = (int)std::min<int64_t>(want, 65535); partial = reinterpret_cast<double*>(p.partial); }
     }
-    if (p.smooth_k) {
-      long long chunk = (p.N + nsplit - 1) / nsplit;
-      chunk = (chunk + 15) / 16 * 16;
-      dim3 grid(nsplit, (unsigned)bh);
-      auto kmean = p.cu_k ? kmean_kernel<T, true> : kmean_kernel<T, false>;
-      e = launch_after_predecessor(kmean, grid, dim3(256), 0, st, reinterpret_cast<const T*>(p.k), p.mean, partial, words,
-                                   (long long)p.N, (long long)p.H, (long long)p.k_strides[0], (long long)p.k_strides[1],
-                                   (long long)p.k_strides[2], nsplit, chunk, (int)p.D, p.cu_k, (long long)p.Tk);
-      if (e != cudaSuccess) return e;
+    long long chunk = (p.N + nsplit - 1) / nsplit;
+    chunk = (chunk + 15) / 16 * 16;
+    const MeanOf<T> of_k = {reinterpret_cast<const T*>(p.k), p.mean, partial, words, p.k_strides[0], p.k_strides[1], p.k_strides[2]};
+    MeanOf<T> of_v = {reinterpret_cast<const T*>(p.v), p.vmean, partial, words + 3 * bh, p.v_strides[0], p.v_strides[1], p.v_strides[2]};
+    auto mean_of = [&](const MeanOf<T>& first, const MeanOf<T>& second, unsigned tensors) {
+      return launch_after_predecessor(p.cu_k ? kmean_kernel<T, true> : kmean_kernel<T, false>, dim3(nsplit, (unsigned)bh, tensors),
+                                      dim3(256), 0, st, first, second, (long long)p.N, (long long)p.H, nsplit, chunk, (int)p.D,
+                                      p.cu_k, (long long)p.Tk);
+    };
+    // V's partial sums go where the staged V factors will be written, if they fit there
+    if (p.smooth_k && p.vmean && (size_t)nsplit * HD * sizeof(double) <= (size_t)p.N_pad * sizeof(float)) {
+      of_v.partial = reinterpret_cast<double*>(p.svp);
+      e = mean_of(of_k, of_v, 2);
+    } else {
+      if (p.smooth_k) e = mean_of(of_k, of_k, 1);
+      if (e == cudaSuccess && p.vmean) e = mean_of(of_v, of_v, 1);
     }
-    if (p.vmean) {
-      long long chunk = (p.N + nsplit - 1) / nsplit;
-      chunk = (chunk + 15) / 16 * 16;
-      dim3 grid(nsplit, (unsigned)bh);
-      auto kmean = p.cu_k ? kmean_kernel<T, true> : kmean_kernel<T, false>;
-      e = launch_after_predecessor(kmean, grid, dim3(256), 0, st, reinterpret_cast<const T*>(p.v), p.vmean, partial, words + 3 * bh,
-                                   (long long)p.N, (long long)p.H, (long long)p.v_strides[0], (long long)p.v_strides[1],
-                                   (long long)p.v_strides[2], nsplit, chunk, (int)p.D, p.cu_k, (long long)p.Tk);
-      if (e != cudaSuccess) return e;
-    }
+    if (e != cudaSuccess) return e;
   }
   const long long total = (a.only_q ? 0 : 2 * (long long)bh * tk) + (long long)a.BHq * tq;
   long long ctas = (long long)sm_count[dev] * QT_MINBLOCKS;
