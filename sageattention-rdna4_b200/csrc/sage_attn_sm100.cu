@@ -48,7 +48,10 @@
 // c_q and sk are applied one after the other instead of as one pre-multiplied factor, a
 // difference of one rounding in a quantity the reference does not pin bit-wise)
 //
-// Every kernel is instantiated twice (template parameter FAST).  The FAST kernels test every key
+// Further instantiations (template parameter ROWS) serve calls with few queries, whose keys are split
+// over CTAs, calls whose query tiles are mostly empty, and heads of up to 64 columns.
+//
+// Every kernel for whole tiles is instantiated twice (template parameter FAST).  The FAST kernels test every key
 // tile against the running row maxima and do not exponentiate a tile whose scores all lie 40
 // exponent units or more below them (its P entries are exact zeros either way); they count what
 // they skip.  The others carry none of that code, and the host chooses between the two sets
@@ -297,6 +300,8 @@ __device__ __forceinline__ void transpose4(uint32_t (&w)[4], int c) {
   }
 }
 
+constexpr uint32_t IDESC_F8_N64 = (1u << 4) | (0u << 7) | (0u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+
 struct AttnKArgs {
   const float *sq, *sk, *svp, *s_fold;
   void* out;
@@ -350,12 +355,18 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
 // elsewhere: 0.035 of the result's 2-norm away from the unsplit kernel, as far as e4m3 goes.)
 // RAGGED and both of these also fold grouped heads and leave out softmax warps without a row; the
 // kernels without either (WHOLE) carry none of that code: it costs their schedule 1 to 6 %.
-enum { WHOLE = 0, RAGGED = 1, SPLIT_MAX = 2, SPLIT_SUM = 3 };
+// NARROW (head_dim up to 64): half of the products' inner and output columns are zeros and are left
+// out, and rescaling and the epilogue touch half the accumulator: 4 x 16 heads x 2 048 130 -> 119 us,
+// 24 x 4 096 192 -> 182, 16 x 16 384 1 583 -> 1 570.  (Not in the kernels with the negligible-tile tests,
+// for packed batches or mostly empty tiles.)
+enum { WHOLE = 0, RAGGED = 1, SPLIT_MAX = 2, SPLIT_SUM = 3, NARROW = 4 };
 template <bool INT8, bool CAUSAL, typename OutT, int NQ, bool FAST, bool VARLEN, int ROWS>
 __global__ void __launch_bounds__(Shape<NQ>::THREADS, Shape<NQ>::CTAS_PER_SM)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const AttnKArgs a) {
   using L = Shape<NQ>;
+  constexpr int QK_STEPS = ROWS == NARROW ? 2 : 4;           // 32 bytes of inner dimension each
+  constexpr uint32_t IDESC_PV = ROWS == NARROW ? IDESC_F8_N64 : IDESC_F8;
   constexpr bool SPLIT = ROWS == SPLIT_MAX || ROWS == SPLIT_SUM;
   constexpr uint32_t OFF_Q = L::OFF_Q, OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_P = L::OFF_P, OFF_SK = L::OFF_SK,
                      OFF_SV = L::OFF_SV, OFF_BAR = L::OFF_BAR, OFF_MISC = L::OFF_MISC;
@@ -421,7 +432,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // an empty second tile keeps its barriers turning).  The others stay out of the loop and of the
   // barriers' counts: their rows of P are never written and their rows of O never read.
   auto live_warps = [&](int g) {
-    if (ROWS == WHOLE) return 8;
+    if (ROWS == WHOLE || ROWS == NARROW) return 8;
     const long long rows = (VARLEN ? Nq_live : a.Nq) - (long long)(q_tile0 + g) * TILE;
     return (int)min(max((rows + 15) / 16, 1LL), 8LL);
   };
@@ -533,7 +544,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < QK_STEPS; ++k)
               mma_ss<INT8>(tmem + L::tmem_s(g), kmajor_sw128_desc(base + OFF_Q + g * TILE_BYTES + 32 * k),
                            kmajor_sw128_desc(base + OFF_K + s * TILE_BYTES + 32 * k), IDESC_QK, k > 0);
             tc_commit(bar(BAR_KE + s));
@@ -571,7 +582,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int k = 0; k < 4; ++k)
               mma_ss<false>(tmem + L::tmem_o(g),
                             kmajor_nosw_desc(base + OFF_P + (g * L::P_BUFS + (jj & (L::P_BUFS - 1))) * TILE_BYTES + 256 * k),
-                            kmajor_sw128_desc(base + OFF_V + s * TILE_BYTES + 32 * k), IDESC_F8,
+                            kmajor_sw128_desc(base + OFF_V + s * TILE_BYTES + 32 * k), IDESC_PV,
                             (jj > 0 || k > 0) ? 1u : 0u);
             tc_commit(bar(BAR_VE + s));
             tc_commit(of_pair(BAR_PV, gb, jj));
@@ -625,7 +636,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < QK_STEPS; ++k)
               mma_ss<INT8>(tmem + L::tmem_s(g), kmajor_sw128_desc(base + OFF_Q + g * TILE_BYTES + 32 * k),
                            kmajor_sw128_desc(base + OFF_K + s * TILE_BYTES + 32 * k), IDESC_QK, k > 0);
             tc_commit(bar(BAR_KE + s));
@@ -653,7 +664,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int k = 0; k < 4; ++k)
               mma_ss<false>(tmem + L::tmem_o(g),
                             kmajor_nosw_desc(base + OFF_P + (g * L::P_BUFS + (jj & (L::P_BUFS - 1))) * TILE_BYTES + 256 * k),
-                            kmajor_sw128_desc(base + OFF_V + s * TILE_BYTES + 32 * k), IDESC_F8,
+                            kmajor_sw128_desc(base + OFF_V + s * TILE_BYTES + 32 * k), IDESC_PV,
                             (jj > 0 || k > 0) ? 1u : 0u);
             tc_commit(bar(BAR_VE + s));
             tc_commit(of_pair(BAR_PV, gb, jj));
@@ -676,7 +687,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int sub = ((warp - 4) >> 2) & 1;                // which 16 lanes of the quarter
       const int r0 = lane >> 2, c = lane & 3;
       const int lane_base = 32 * quarter + 16 * sub;
-      if (ROWS == WHOLE || lane_base < 16 * live_warps(g)) {
+      if (ROWS == WHOLE || ROWS == NARROW || lane_base < 16 * live_warps(g)) {
       const int n_tiles = tiles_of(g);
       const int rowA = lane_base + r0, rowB = rowA + 8;     // this thread's two query rows of the tile
       const long long q_rowA = (long long)q_tile * TILE + rowA, q_rowB = q_rowA + 8;
@@ -938,16 +949,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (rescale) {
           const float2 aA2 = make_float2(alphaA, alphaA), aB2 = make_float2(alphaB, alphaB);
           uint32_t o[64];
-          tmem_ld_16x256b_x16(t_o, o);
+          if (ROWS == NARROW) tmem_ld_16x256b_x8(t_o, o); else tmem_ld_16x256b_x16(t_o, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
+          for (int i = 0; i < (ROWS == NARROW ? 8 : 16); ++i) {
             const float2 ra = __fmul2_rn(make_float2(__uint_as_float(o[4 * i + 0]), __uint_as_float(o[4 * i + 1])), aA2);
             const float2 rb = __fmul2_rn(make_float2(__uint_as_float(o[4 * i + 2]), __uint_as_float(o[4 * i + 3])), aB2);
             o[4 * i + 0] = __float_as_uint(ra.x); o[4 * i + 1] = __float_as_uint(ra.y);
             o[4 * i + 2] = __float_as_uint(rb.x); o[4 * i + 3] = __float_as_uint(rb.y);
           }
-          tmem_st_16x256b_x16(t_o, o);
+          if (ROWS == NARROW) tmem_st_16x256b_x8(t_o, o); else tmem_st_16x256b_x16(t_o, o);
           tmem_st_wait();
         }
         fence_async_smem();
@@ -1017,14 +1028,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         const float* vm = (a.vmean != nullptr) ? a.vmean + (size_t)bh_kv * HD + 2 * c : nullptr;
         uint32_t o[64];
-        tmem_ld_16x256b_x16(t_o, o);
+        if (ROWS == NARROW) tmem_ld_16x256b_x8(t_o, o); else tmem_ld_16x256b_x16(t_o, o);
         tmem_ld_wait();
         // A thread holds channels 8i + 2c, 8i + 2c + 1.  The four threads of a row exchange words, so
         // that each writes whole 16-byte blocks and a warp's store covers 64 contiguous bytes of a
         // row instead of 16 (32 stores of 4 bytes became 8 of 16): 40 heads, 16 384 queries of
         // 512 keys 235 -> 218 us, 48 x 2 048 x 2 048 113 -> 108, 48 x 8 771 x 8 771 1 596 -> 1 558.
 #pragma unroll
-        for (int i4 = 0; i4 < 4; ++i4) {
+        for (int i4 = 0; i4 < (ROWS == NARROW ? 2 : 4); ++i4) {
           uint32_t wa[4], wb[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -1291,6 +1302,7 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
   // slots of the longest length at most.
   if (varlen && p.plan)
     grid = dim3((unsigned)(std::min<int64_t>(p.Tq / TILE + p.B, p.B * (int64_t)q_tiles) * p.Hq));
+  const bool narrow = p.D <= 64 && !fast;
   ka.skip_log2 = skip;
   ka.skipped = fast ? p.skipped : nullptr;
   if (n_split > 1) {
@@ -1318,6 +1330,8 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
 #define SAGE_LAUNCH(I8, C, T)                                                                          \
   e = varlen ? launch_inst<I8, C, T, 1, false, true>(mq, mk, mv, ka, grid, st) :                       \
       ragged ? launch_inst<I8, false, T, 1, false, false, RAGGED>(mq, mk, mv, ka, grid, st) :          \
+      narrow ? (two ? launch_inst<I8, C, T, 2, false, false, NARROW>(mq, mk, mv, ka, grid, st)           \
+                    : launch_inst<I8, C, T, 1, false, false, NARROW>(mq, mk, mv, ka, grid, st)) :        \
       two ? (fast ? launch_inst<I8, C, T, 2, true>(mq, mk, mv, ka, grid, st)                           \
                   : launch_inst<I8, C, T, 2, false>(mq, mk, mv, ka, grid, st))                         \
           : (fast ? launch_inst<I8, C, T, 1, true>(mq, mk, mv, ka, grid, st)                           \
