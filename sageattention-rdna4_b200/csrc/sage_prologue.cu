@@ -899,33 +899,52 @@ static bool make_map4(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, i
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename T, bool INT8>
-static cudaError_t launch_short(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const QuantArgs& a,
-                                const ShortArgs& sa, int64_t tiles_k, cudaStream_t st) {
-  auto kern = quant_short_kernel<T, INT8>;
-  static bool opted_in[64] = {false};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64 || !opted_in[dev]) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)short_smem::BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) opted_in[dev] = true;
-  }
-  const unsigned ctas = (unsigned)tiles_k;                              // per cluster
-  const int64_t per_cluster = (int64_t)ctas * 2;                        // Q tiles a cluster takes
-  const unsigned clusters = (unsigned)(sa.kv_clusters + (sa.items_q + per_cluster - 1) / per_cluster);
+static cudaLaunchConfig_t short_config(cudaLaunchAttribute attr[2], unsigned clusters, unsigned ctas, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(clusters * ctas); cfg.blockDim = dim3(512); cfg.dynamicSmemBytes = short_smem::BYTES; cfg.stream = st;
-  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = ctas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, a, sa);
+  return cfg;
+}
+
+// The largest cluster of quant_short_kernel that the device can place (16, 8 or none; a partition of
+// a GPU may have fewer SMs side by side), asked once per device together with the opt-ins.
+template <typename T, bool INT8>
+static cudaError_t short_cluster_limit(int dev, int* limit) {
+  static int known[64] = {0};                                           // limit + 1
+  if (known[dev] == 0) {
+    auto kern = quant_short_kernel<T, INT8>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)short_smem::BYTES);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    int best = 0;
+    for (int ctas = SHORT_CTAS; ctas >= 8 && best == 0; ctas /= 2) {
+      cudaLaunchAttribute attr[2];
+      cudaLaunchConfig_t cfg = short_config(attr, 1, (unsigned)ctas, nullptr);
+      cfg.attrs = attr + 1; cfg.numAttrs = 1;                           // the cluster size alone
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) best = ctas;
+      else (void)cudaGetLastError();
+    }
+    known[dev] = best + 1;
+  }
+  *limit = known[dev] - 1;
+  return cudaSuccess;
+}
+
+template <typename T, bool INT8>
+static cudaError_t launch_short(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const QuantArgs& a,
+                                const ShortArgs& sa, int64_t tiles_k, cudaStream_t st) {
+  const unsigned ctas = (unsigned)tiles_k;                              // per cluster
+  const int64_t per_cluster = (int64_t)ctas * 2;                        // Q tiles a cluster takes
+  const unsigned clusters = (unsigned)(sa.kv_clusters + (sa.items_q + per_cluster - 1) / per_cluster);
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = short_config(attr, clusters, ctas, st);
+  return cudaLaunchKernelEx(&cfg, quant_short_kernel<T, INT8>, mq, mk, mv, a, sa);
 }
 
 template <typename T>
@@ -981,7 +1000,12 @@ static cudaError_t launch_typed(const PrologueParams& p, cudaStream_t st) {
   // tokens 58.2 / 62.3 (576), 1 100 tokens 63.3 / 69.1 (648), 1 536 tokens 100 / 95 (864), 2 048
   // tokens 169 / 154 (1 152); 8 heads of 2 048 tokens 50.4 / 56.4 (192); 40 heads, 8 192 queries of
   // 1 024 keys 236 / 231 (1 600).
-  if (!varlen && tk <= SHORT_CTAS && bh * tk + (a.BHq * tq + 1) / 2 <= 5 * (int64_t)sm_count[dev]) {
+  int most_ctas = 0;
+  if (!varlen && tk <= SHORT_CTAS) {
+    e = (p.qk_mode == 0) ? short_cluster_limit<T, true>(dev, &most_ctas) : short_cluster_limit<T, false>(dev, &most_ctas);
+    if (e != cudaSuccess) return e;
+  }
+  if (!varlen && tk <= most_ctas && bh * tk + (a.BHq * tq + 1) / 2 <= 5 * (int64_t)sm_count[dev]) {
     ShortArgs sa;
     sa.mean = p.mean; sa.vmean = p.vmean; sa.words = words; sa.n_words = (int)CtrlHeader::words(bh); sa.kv_clusters = (int)bh;
     sa.items_q = a.qm ? 0 : a.BHq * tq;      // Q tiles that need K's mean (for the LSE) follow in a launch of their own
