@@ -292,7 +292,7 @@ int sage_attn_fwd_reported(const void* q8, const float* sq, const void* k8, cons
  * A sequence without queries costs nothing; one with queries and no keys gets rows of zeros.
  * The arrays are not validated (that would need them on the host); the kernels clamp every start
  * and end to the packed token counts, so that no access leaves q, k, v or out whatever they hold.
- * The kernels run the one-tile shape without the negligible-tile tests.  Status word and errors as
+ * The kernels run without the negligible-tile tests.  Status word and errors as
  * for sage_attention (the layout is sage_workspace_layout_ex(n_seq, Hq, Hkv, max_q, max_k)). */
 int sage_attention_varlen(const void* q, const void* k, const void* v, void* out,
                           const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,

@@ -391,7 +391,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // the blockIdx.x-th query tile that exists: sequences in the order of the work list (longest
     // first), head by head; 32 of the list's prefix sums at a time
     const int x = (int)blockIdx.x, hq = (int)a.Hq;
-    const int* pre = a.plan + a.n_seq + 1;
+    const int* pre = a.plan + (NQ == 1 ? 1 : 4) * (a.n_seq + 1);       // query tiles, or pairs of them
     if (x >= pre[a.n_seq] * hq) return;
     int s = 0;
     for (;; s += 32) {
@@ -400,7 +400,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     const int rem = x - pre[s] * hq, per = pre[s + 1] - pre[s];
     bh = a.plan[s] * hq + rem / per;
-    q_tile0 = CAUSAL ? per - 1 - rem % per : rem % per;
+    q_tile0 = NQ * (CAUSAL ? per - 1 - rem % per : rem % per);
   }
   const int bh_kv = (int)((bh / a.Hq) * a.H + (bh % a.Hq) / a.group);   // its (batch, K/V head)
   // Key tiles query tile g visits: all of them, or when causal those up to its diagonal (a causal
@@ -1256,8 +1256,7 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
       sm_count[dev] = 148;
     sms = sm_count[dev];
   }
-  // A packed batch runs on the one-tile kernels without the negligible-tile tests: its sequences
-  // differ in length, and the smaller unit of work evens them out.
+  // A packed batch runs on kernels without the negligible-tile tests.
   const bool varlen = p.cu_q != nullptr;
   const int forced = g_force_tiles_per_cta.load(std::memory_order_relaxed);
   bool two = choose_tiles_per_cta((p.Nq + TILE - 1) / TILE, p.B * p.Hq, p.causal != 0, sms) == 2;
@@ -1266,7 +1265,10 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
   // 12.7 / 14.4; 2 x 24 x 1 000 x 1 000 39.4 / 45.5; but 48 x 2 048 x 2 048 (16 key tiles) 121 / 118.
   if (p.N_pad <= 8 * TILE) two = false;
   if (forced != 0) two = (forced == 2);
-  if (varlen) two = false;
+  // Packed batches: two tiles per CTA once there are about ten rounds of such CTAs, so that what is
+  // left over at the end (CTAs come longest first) does not weigh: 48 heads, 36 k tokens in eleven sequences of
+  // 512 .. 8 192 (46 rounds), whole call 4 369 us with one tile, 4 216 with two.
+  if (varlen) two = p.plan && (forced ? forced == 2 : p.Tq / (2 * TILE) * p.Hq >= 10 * (int64_t)sms);
   // Which of the two sets of kernels: with the negligible-tile tests (the default) or without.
   // The threshold hook at 0 and the caller's `no_fast_path` both select the plain set.
   const float skip = g_skip_log2.load(std::memory_order_relaxed);
@@ -1301,7 +1303,8 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
   // With a work list the grid covers the tiles that sequences of Tq tokens in all can have, in
   // slots of the longest length at most.
   if (varlen && p.plan)
-    grid = dim3((unsigned)(std::min<int64_t>(p.Tq / TILE + p.B, p.B * (int64_t)q_tiles) * p.Hq));
+    grid = dim3((unsigned)((two ? std::min<int64_t>(p.Tq / (2 * TILE) + p.B, p.B * (int64_t)((q_tiles + 1) / 2))
+                                : std::min<int64_t>(p.Tq / TILE + p.B, p.B * (int64_t)q_tiles)) * p.Hq));
   const bool narrow = p.D <= 64 && !fast;
   ka.skip_log2 = skip;
   ka.skipped = fast ? p.skipped : nullptr;
@@ -1328,7 +1331,8 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
   const int key = (p.qk_mode == 0 ? 4 : 0) | (p.causal ? 2 : 0) | (p.out_dtype == 0 ? 1 : 0);
   cudaError_t e;
 #define SAGE_LAUNCH(I8, C, T)                                                                          \
-  e = varlen ? launch_inst<I8, C, T, 1, false, true>(mq, mk, mv, ka, grid, st) :                       \
+  e = varlen ? (two ? launch_inst<I8, C, T, 2, false, true>(mq, mk, mv, ka, grid, st)                  \
+                    : launch_inst<I8, C, T, 1, false, true>(mq, mk, mv, ka, grid, st)) :               \
       ragged ? launch_inst<I8, false, T, 1, false, false, RAGGED>(mq, mk, mv, ka, grid, st) :          \
       narrow ? (two ? launch_inst<I8, C, T, 2, false, false, NARROW>(mq, mk, mv, ka, grid, st)           \
                     : launch_inst<I8, C, T, 1, false, false, NARROW>(mq, mk, mv, ka, grid, st)) :        \

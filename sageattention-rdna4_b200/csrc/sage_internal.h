@@ -35,7 +35,7 @@ struct PrologueParams {
 
 // Work list of a packed batch (see plan_packed_kernel); batches of more sequences go without.
 constexpr int PLAN_MAX_SEQS = 512;
-inline size_t plan_bytes(int64_t B) { return B <= PLAN_MAX_SEQS ? (size_t)4 * (size_t)(B + 1) * sizeof(int) : 0; }
+inline size_t plan_bytes(int64_t B) { return B <= PLAN_MAX_SEQS ? (size_t)5 * (size_t)(B + 1) * sizeof(int) : 0; }
 
 struct AttnParams {
   const void *q8, *k8, *v8t;

@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(256) clear_ctrl_kernel(unsigned* __restrict__ 
 }
 
 // The same for a packed batch, and the batch's work list: the sequences ordered by their work,
-// longest first, and in that order the prefix sums of their query tiles, key tiles and fold items
-// (plan: four arrays of B + 1 words).  The kernels behind it then draw only tiles that exist; in
+// longest first, and in that order the prefix sums of their query tiles, key tiles, fold items and
+// pairs of query tiles (plan: five arrays of B + 1 words).  The kernels behind it then draw only tiles that exist; in
 // slots of the longest length, 59 % of the quantiser's items and of the attention grid were empty
 // in a batch of eleven sequences of 512 .. 8 192 tokens.  One block: a few microseconds for up to
 // PLAN_MAX_SEQS sequences.
@@ -55,7 +55,7 @@ plan_packed_kernel(unsigned* __restrict__ words, int n, int* __restrict__ plan, 
                    const int* __restrict__ cu_q, const int* __restrict__ cu_k, long long Tq, long long Tk,
                    long long Nq, long long Nk) {
   __shared__ long long s_work[PLAN_MAX_SEQS];
-  __shared__ int s_pre[3][PLAN_MAX_SEQS];
+  __shared__ int s_pre[4][PLAN_MAX_SEQS];
   wait_for_predecessor();
   allow_successor();
   const int tid = threadIdx.x;
@@ -69,28 +69,29 @@ plan_packed_kernel(unsigned* __restrict__ words, int n, int* __restrict__ plan, 
   if (tid < B) { tq = tiles(cu_q, Tq, Nq); tk = tiles(cu_k, Tk, Nk); }
   const long long work = (long long)tq * tk;
   s_work[tid] = work;
-  s_pre[0][tid] = 0; s_pre[1][tid] = 0; s_pre[2][tid] = 0;
+  s_pre[0][tid] = 0; s_pre[1][tid] = 0; s_pre[2][tid] = 0; s_pre[3][tid] = 0;
   __syncthreads();
   if (tid < B) {
     int rank = 0;
     for (int i = 0; i < B; ++i) rank += (s_work[i] > work || (s_work[i] == work && i < tid)) ? 1 : 0;
     plan[rank] = tid;
     s_pre[0][rank] = tq; s_pre[1][rank] = tk; s_pre[2][rank] = (tk * TILE + FOLD_KEYS - 1) / FOLD_KEYS;
+    s_pre[3][rank] = (tq + 1) / 2;
   }
   __syncthreads();
-  for (int off = 1; off < PLAN_MAX_SEQS; off <<= 1) {        // inclusive scan of the three arrays
-    int v[3];
+  for (int off = 1; off < PLAN_MAX_SEQS; off <<= 1) {        // inclusive scan of the four arrays
+    int v[4];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) v[a] = (tid >= off) ? s_pre[a][tid - off] : 0;
+    for (int a = 0; a < 4; ++a) v[a] = (tid >= off) ? s_pre[a][tid - off] : 0;
     __syncthreads();
 #pragma unroll
-    for (int a = 0; a < 3; ++a) s_pre[a][tid] += v[a];
+    for (int a = 0; a < 4; ++a) s_pre[a][tid] += v[a];
     __syncthreads();
   }
-  if (tid < 3) plan[(tid + 1) * (B + 1)] = 0;
+  if (tid < 4) plan[(tid + 1) * (B + 1)] = 0;
   if (tid < B)
 #pragma unroll
-    for (int a = 0; a < 3; ++a) plan[(a + 1) * (B + 1) + tid + 1] = s_pre[a][tid];
+    for (int a = 0; a < 4; ++a) plan[(a + 1) * (B + 1) + tid + 1] = s_pre[a][tid];
 }
 
 // ------------------------------------------------------------------------------------------------

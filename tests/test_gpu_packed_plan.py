@@ -6,16 +6,18 @@ import pytest
 import torch
 
 import sageattention
+from sageattention import _native
 from sageattention import b200_backend as be
 
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("shape", [0, 2])
 @pytest.mark.parametrize("n_seq,hq,hkv,causal,longest", [
     (2, 3, 1, False, 1500), (33, 2, 2, True, 300), (64, 4, 2, False, 129),
     (512, 2, 1, False, 140), (513, 2, 1, True, 140),           # the longest list and the first batch without one
 ])
-def test_work_list_against_single_calls(n_seq, hq, hkv, causal, longest):
+def test_work_list_against_single_calls(shape, n_seq, hq, hkv, causal, longest):
     rng = random.Random(n_seq)
     lens = [rng.choice([0, 1, 127, 128, 129, rng.randint(1, longest)]) for _ in range(n_seq)]
     lens = [min(n, longest) for n in lens]
@@ -25,7 +27,11 @@ def test_work_list_against_single_calls(n_seq, hq, hkv, causal, longest):
     q, k, v = (torch.randn(total, h, 128, generator=g, device="cuda").half() for h in (hq, hkv, hkv))
     k += torch.randn(1, hkv, 128, generator=g, device="cuda").half()
     cu = torch.tensor([sum(lens[:i]) for i in range(n_seq + 1)], dtype=torch.int32, device="cuda")
-    out = sageattention.sageattn_varlen(q, k, v, cu, cu, longest, longest, is_causal=causal)
+    _native.load().sage_debug_tiles_per_cta(shape)             # 2: pairs of query tiles
+    try:
+        out = sageattention.sageattn_varlen(q, k, v, cu, cu, longest, longest, is_causal=causal)
+    finally:
+        _native.load().sage_debug_tiles_per_cta(0)
     torch.cuda.synchronize()
     be.check()
     at = 0
