@@ -344,9 +344,9 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, fl
 // (ceil(Nq/256), B*Hq), block 640, one CTA per SM.
 // ------------------------------------------------------------------------------------------------
 // VARLEN: a packed batch.  a.Nq, a.N_pad are the capacity of a sequence's slot in the quantised
-// operands, the grid is sized for the longest sequence allowed; each sequence's own lengths and the
-// first row of its output come from cu_q / cu_k, and a CTA whose query tile lies past its
-// sequence's end returns at once.
+// operands; each sequence's own lengths and the first row of its output come from cu_q / cu_k.  With a
+// work list the x-th CTA takes the x-th query tile that exists; without one the grid is sized for the
+// longest sequence allowed and a CTA whose query tile lies past its sequence's end returns at once.
 // SPLIT: a share of the key range per CTA (blockIdx.x = query tile * splits + share), in two launches.
 // SPLIT_MAX only finds each row's score maximum in the share (part_max).  SPLIT_SUM starts from the
 // maximum over the shares before its own, so that its running maxima, and with them the e4m3 codes of

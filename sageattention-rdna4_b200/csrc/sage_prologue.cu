@@ -1,7 +1,7 @@
 // Quantisation prologue for B200: sequence mean of K (smooth_k; of V too with smooth_v), then one
 // persistent, TMA-fed pass over the 128-token tiles of K, V and Q that writes the int8 / e4m3
 // codes, the per-token scales and V transposed, and closes with the fold of the per-head S and its
-// staged factor.
+// staged factor.  Short calls take one launch of clusters instead (quant_short_kernel).
 //
 // Arithmetic contract (reference: kernels/hip/h34_prologue.hip:116-211,259-282;
 // kernels/hip/sk1_t6i.hip:104-117; kernels/hip/sk1_t4a1sb.hip:89-100;
