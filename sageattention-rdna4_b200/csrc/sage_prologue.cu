@@ -768,12 +768,21 @@ quant_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"((int)(tile * TILE)), "r"(h), "r"(b) : "memory");
   };
-  // bounded wait; a thread that gives up reports it and goes on, so that no barrier misses it
+  // bounded wait; a thread that gives up reports it and goes on, so that no barrier misses it.  It does
+  // not wait a second time, and it stays a moment before it leaves: the copy may still arrive, and this
+  // CTA's shared memory must not be another's by then.
+  bool lost = false;
   auto landed = [&]() {
-    if (qt_try_wait(bar, 0)) return;
+    if (lost || qt_try_wait(bar, 0)) return;
     const long long t0 = clock64();
     while (!qt_try_wait(bar, 0))
-      if (clock64() - t0 > QT_WAIT_CYCLES) { atomicOr(a.status, 1); if (a.status2) atomicOr(a.status2, 8); return; }
+      if (clock64() - t0 > QT_WAIT_CYCLES) { atomicOr(a.status, 1); if (a.status2) atomicOr(a.status2, 8); lost = true; return; }
+  };
+  auto before_leaving = [&]() {
+    if (lost) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < 400000) { }
+    }
   };
   uint8_t* stage = gbase + (uint32_t)grp * QT_STAGE_BYTES;
   auto half_sync = [&]() { if (grp == 0) tile_sync<1>(); else tile_sync<2>(); };
@@ -786,6 +795,7 @@ quant_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (gt == 0) load(&tm_q, tile, bh, a.Hq);
     landed();
     quant_q_tile<T, INT8>(a, stage, bh, tile * TILE, a.Nq, c, r0);
+    before_leaving();
     return;
   }
 
@@ -865,6 +875,7 @@ quant_short_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (rank == 0 && gt == 0) a.s_fold[bh] = S;
     if (gt < TILE) a.svp[(size_t)bh * a.N_pad + n_base + gt] = __fmul_rn(__fdiv_rn(sv_s[gt], S), F8_MAX);
   }
+  before_leaving();
 }
 
 // ------------------------------------------------------------------------------------------------
