@@ -245,9 +245,12 @@ int sage_workspace_layout_ex(int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int
 /* sage_attention_ex, sage_attention_varlen and sage_attn_fwd_ex with one more argument.
  * `status_host` (may be null) is a 4-byte word of pinned host memory that the device can write
  * (cudaHostAlloc / cudaHostRegister).  When a bounded wait of the call has run out, the attention
- * kernel writes the call's status word there; a call that succeeds writes nothing, so that a host
- * learns of a failure without a copy behind every call.  The word must stay allocated until the
- * call has finished; a captured call keeps using it in every replay. */
+ * kernel writes the call's status word there, once, and adds 0x100 (SAGE_STATUS_REPORTED) to the
+ * word in device memory, so that the host may clear its word while the failed call still ends; a
+ * call that succeeds writes nothing, so that a host learns of a failure without a copy behind every
+ * call.  The word must stay allocated until the call has finished; a captured call keeps using it in
+ * every replay. */
+#define SAGE_STATUS_REPORTED 0x100
 int sage_attention_reported(const void* q, const void* k, const void* v, void* out, float* lse,
                             void* workspace, size_t workspace_bytes,
                             int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int64_t head_dim,

@@ -112,7 +112,7 @@ enum Bar { BAR_Q = 0, BAR_KF = 1, BAR_KE = 3, BAR_VF = 5, BAR_VE = 7, BAR_SF = 9
            BAR_PF = 11, BAR_PV = 13, BAR_PER_TILE = 6, BAR_COUNT = 21 };
 static_assert(BAR_COUNT * 8 <= 192, "barrier area");
 
-enum { ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_SOFTMAX = 4 };
+enum { ST_TIMEOUT_PRODUCER = 1, ST_TIMEOUT_MMA = 2, ST_TIMEOUT_SOFTMAX = 4, ST_REPORTED = 0x100 };
 
 constexpr long long WAIT_CYCLES = 4000000000LL;      // about two seconds of SM clock
 
@@ -1067,10 +1067,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   if (*cta_abort) {
-    // The host sees a failure through this one word; a call that succeeds writes nothing.  (Every
-    // thread writes it: an index kept to this point costs the kernels spilled registers.)
+    // The host sees a failure through this one word; a call that succeeds writes nothing.  One thread
+    // of the call writes it, the first to mark the status word as reported: the host clears the word
+    // when it raises, possibly while CTAs of the failed call still end.  (Every thread tries: an index
+    // kept to this point costs the kernels spilled registers.)
     if (a.status_host != nullptr) {
-      *reinterpret_cast<volatile int32_t*>(a.status_host) = *reinterpret_cast<volatile int32_t*>(a.status);
+      const int32_t seen = atomicOr(a.status, (int32_t)ST_REPORTED);
+      if (!(seen & ST_REPORTED)) *reinterpret_cast<volatile int32_t*>(a.status_host) = seen;
     }
     const long long t0 = clock64();
     while (clock64() - t0 < 400000) { }

@@ -17,6 +17,7 @@ LIB_PATH = os.path.join(_HERE, "libsage_b200.so")
 SAGE_F16, SAGE_BF16 = 0, 1
 SAGE_QK_INT8, SAGE_QK_E4M3 = 0, 1
 SAGE_QK_NO_FAST_PATH = 0x100
+SAGE_STATUS_REPORTED = 0x100
 SAGE_E_ARG, SAGE_E_UNSUPPORTED, SAGE_E_CUDA, SAGE_E_WORKSPACE = -1, -2, -3, -4
 
 _I64 = ctypes.c_int64

@@ -223,8 +223,8 @@ def attn_launch(pq: Dict[str, torch.Tensor], out: torch.Tensor, is_causal: bool,
 # undefined.  The reference raises in such a case only in its strict mode and otherwise falls back
 # (sageattention/sk1_backend/__init__.py:1022-1027,1114-1123); this path has no fallback, so the
 # failure must reach the caller.  The attention kernel of a call that failed writes the status word
-# into a word of pinned host memory (one that succeeds writes nothing, so nothing follows a call on
-# the stream); the next call on that stream, `check()` or `status()` looks at the host word and
+# into a word of pinned host memory, once (one that succeeds writes nothing, so nothing follows a call
+# on the stream); the next call on that stream, `check()` or `status()` looks at the host word and
 # raises RuntimeError when it is non-zero.
 # SAGEATTN_B200_STRICT=1 synchronises after every call and checks at once;
 # SAGEATTN_B200_WATCH=0 switches the report off.
@@ -683,7 +683,7 @@ def last_status(q_like: torch.Tensor, b: int, h: int, n: int, hkv: Optional[int]
     if st.shape != want:
         raise RuntimeError("last_status: the last call on this stream had shape %r, not %r" % (st.shape, want))
     stream.synchronize()
-    return int(st.ws[st.status_off: st.status_off + 4].view(torch.int32).item())
+    return int(st.ws[st.status_off: st.status_off + 4].view(torch.int32).item()) & ~_native.SAGE_STATUS_REPORTED
 
 
 def status() -> dict:

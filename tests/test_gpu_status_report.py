@@ -46,6 +46,27 @@ def test_the_status_word_is_reported_to_the_host(shape, causal):
     assert host.item() == 0 and status.item() == 0 and torch.isfinite(out).all() and not (out == 7.0).any()
 
 
+def test_a_failure_is_reported_once():
+    """The host clears its word when it raises, possibly before the last CTAs of the failed call have
+    started: those see the status word that the first ones left and do not report it again."""
+    lib = _native.load()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = (torch.randn(1, 2, 300, 128, generator=g, device="cuda").half() for _ in range(3))
+    pq = be.quant_qkv(q, k, v)
+    out = torch.full_like(q, 7.0)
+    host = torch.zeros(1, dtype=torch.int32).pin_memory()
+    status = torch.full((1,), 2, dtype=torch.int32, device="cuda")
+    for expected in (2, 0):                                    # the CTAs that come first, and those that come late
+        host.zero_()
+        assert lib.sage_attn_fwd_reported(
+            *(pq[x].data_ptr() for x in ("q8", "sq", "k8", "sk", "v8t", "svp", "S")), out.data_ptr(), None, None, None,
+            1, 2, 2, 300, 300, pq["n_pad"], 128, _native.strides3(*out.stride()[:3]), 0, 128 ** -0.5, 0, 0,
+            status.data_ptr(), host.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert host.item() == expected
+        assert status.item() == 2 | _native.SAGE_STATUS_REPORTED and (out == 7.0).all()
+
+
 def test_status_host_must_be_aligned():
     lib = _native.load()
     buf = (ctypes.c_char * 4096)()
