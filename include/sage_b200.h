@@ -162,7 +162,8 @@ int sage_status_mirror(const int32_t* status_dev, int32_t* status_host, int word
 /* Test hook (one process-wide atomic word): the attention kernel has two shapes, one or two
  * 128-query tiles per CTA, and picks the one it expects to finish sooner for the call's size.
  * n = 1 or 2 forces that shape for later launches from any thread, anything else restores the
- * automatic choice.  Both shapes give bit-identical results. */
+ * automatic choice.  Both shapes give bit-identical results.  A call with a forced shape never splits
+ * its keys. */
 void sage_debug_tiles_per_cta(int n);
 
 /* Test hook (one process-wide atomic word): threshold of the attention kernel's negligible-tile
@@ -174,9 +175,26 @@ void sage_debug_tiles_per_cta(int n);
  * kernels/hip/sk1_t6i.hip:162-279); a negative value restores the default. */
 void sage_debug_skip_threshold(float log2_units);
 
-/* The shape the attention kernel takes, left to itself, for B x Hq heads of Nq queries on a device
- * with sm_count SMs: 1 or 2 query tiles per CTA (0 for bad arguments).  Host arithmetic only. */
+/* The rounds rule behind the choice of shape: 1 or 2 query tiles per CTA for B x Hq heads of Nq
+ * queries on a device with sm_count SMs (0 for bad arguments).  It knows nothing of the keys; calls of
+ * up to 1 024 keys, packed batches and calls whose keys are split do not follow it.
+ * sage_attention_form says what a call takes.  Host arithmetic only. */
 int sage_attention_tiles_per_cta(int64_t B, int64_t Hq, int64_t Nq, int causal, int sm_count);
+
+/* The form in which the attention kernel serves a whole call (sage_attention and its variants with a
+ * workspace of sage_workspace_bytes_ex bytes, no test hook set) on a device with sm_count SMs; the launch
+ * itself asks the same function.  Host arithmetic only.
+ *   packed_q   0 for a fixed-length call; else the call is a packed batch of B sequences with this
+ *              many query tokens in all, of at most Nq queries and Nk keys each
+ *   plain      non-zero for a call with SAGE_QK_NO_FAST_PATH
+ *   form       [0] 128-query tiles per CTA: 1 or 2
+ *              [1] shares into which every head's keys are split (1: not split; merging the shares
+ *                  sums in another order, see sage_attention_ex)
+ *              [2] query heads of a group that share query tiles (1: none)
+ *              [3] 1 if the kernels test key tiles for negligible scores
+ * Returns the number of entries written (4) or an error code. */
+int sage_attention_form(int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int64_t packed_q,
+                        int causal, int plain, int sm_count, int form[4]);
 
 /* Bytes of workspace `sage_attention` needs for one call (all intermediates + ctrl + status). */
 size_t sage_workspace_bytes(int64_t B, int64_t H, int64_t N);

@@ -1243,10 +1243,32 @@ size_t split_scratch_bytes(int64_t B, int64_t Hq, int64_t H, int64_t Nq, int64_t
 // know where a row belongs), and softmax warps without a row stay idle.  Taken when that leaves
 // out a tenth of the softmax warps or more (48 x 288 x 288: 12.7 -> 11.4 us); full tiles lose 1 to
 // 2 % in those kernels (48 x 4 096 x 4 096: 391 -> 396 us).
-static bool mostly_empty_tiles(const AttnParams& p) {
-  const int64_t rows = p.Nq * (p.Hq / p.H);
-  const int64_t warps = 8 * p.Hq * ((p.Nq + TILE - 1) / TILE), live = p.H * ((rows + 15) / 16);
+static bool mostly_empty_tiles(const AttnShape& c) {
+  const int64_t rows = c.Nq * (c.Hq / c.H);
+  const int64_t warps = 8 * c.Hq * ((c.Nq + TILE - 1) / TILE), live = c.H * ((rows + 15) / 16);
   return rows <= ((int64_t)1 << 30) && 10 * live <= 9 * warps;
+}
+
+AttnForm choose_form(const AttnShape& c, int sms) {
+  const bool varlen = c.packed_q > 0, short_loop = c.N <= 8 * TILE;
+  AttnForm f;
+  // A loop over few key tiles is mostly start and end of a CTA, which only a second CTA on the SM
+  // hides: 40 heads x 16 384 queries x 512 keys 235 us with one tile, 265 with two; 48 x 288 x 288
+  // 12.7 / 14.4; 2 x 24 x 1 000 x 1 000 39.4 / 45.5; but 48 x 2 048 x 2 048 (16 key tiles) 121 / 118.
+  f.two = !short_loop && choose_tiles_per_cta((c.Nq + TILE - 1) / TILE, c.B * c.Hq, c.causal != 0, sms) == 2;
+  if (c.forced != 0) f.two = (c.forced == 2);
+  // Packed batches: two tiles per CTA once there are about ten rounds of such CTAs, so that what is
+  // left over at the end (CTAs come longest first) does not weigh: 48 heads, 36 k tokens in eleven sequences of
+  // 512 .. 8 192 (46 rounds), whole call 4 369 us with one tile, 4 216 with two.
+  if (varlen) f.two = c.work_list && (c.forced ? c.forced == 2 : c.packed_q / (2 * TILE) * c.Hq >= 10 * (int64_t)sms);
+  // Neither a packed batch nor a loop over few key tiles takes the negligible-tile tests (most of such a
+  // CTA's time is its start and end).
+  f.fast = c.tests && !varlen && !short_loop;
+  f.splits = (c.scratch && !c.causal && !varlen && c.forced == 0)
+                 ? key_splits(c.B, c.Hq, c.H, c.Nq, c.N, std::min(sms, SPLIT_SIZING_SMS)) : 1;
+  f.ragged = f.splits > 1 || (!c.causal && !varlen && !f.fast && !f.two && mostly_empty_tiles(c));
+  f.fold = f.ragged ? (int)(c.Hq / c.H) : 1;
+  return f;
 }
 
 cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char** why) {
@@ -1259,28 +1281,14 @@ cudaError_t launch_attention(const AttnParams& p_in, cudaStream_t st, const char
       sm_count[dev] = 148;
     sms = sm_count[dev];
   }
-  // A packed batch runs on kernels without the negligible-tile tests.
   const bool varlen = p.cu_q != nullptr;
-  const int forced = g_force_tiles_per_cta.load(std::memory_order_relaxed);
-  bool two = choose_tiles_per_cta((p.Nq + TILE - 1) / TILE, p.B * p.Hq, p.causal != 0, sms) == 2;
-  // A loop over few key tiles is mostly start and end of a CTA, which only a second CTA on the SM
-  // hides: 40 heads x 16 384 queries x 512 keys 235 us with one tile, 265 with two; 48 x 288 x 288
-  // 12.7 / 14.4; 2 x 24 x 1 000 x 1 000 39.4 / 45.5; but 48 x 2 048 x 2 048 (16 key tiles) 121 / 118.
-  if (p.N_pad <= 8 * TILE) two = false;
-  if (forced != 0) two = (forced == 2);
-  // Packed batches: two tiles per CTA once there are about ten rounds of such CTAs, so that what is
-  // left over at the end (CTAs come longest first) does not weigh: 48 heads, 36 k tokens in eleven sequences of
-  // 512 .. 8 192 (46 rounds), whole call 4 369 us with one tile, 4 216 with two.
-  if (varlen) two = p.plan && (forced ? forced == 2 : p.Tq / (2 * TILE) * p.Hq >= 10 * (int64_t)sms);
   // Which of the two sets of kernels: with the negligible-tile tests (the default) or without.
   // The threshold hook at 0 and the caller's `no_fast_path` both select the plain set.
   const float skip = g_skip_log2.load(std::memory_order_relaxed);
-  // (Nor do loops over few key tiles take the tests: most of such a CTA's time is its start and end.)
-  const bool fast = !p.no_fast_path && skip > 0.f && !varlen && p.N_pad > 8 * TILE;
-  const int n_split = (p.part && !p.causal && !varlen && forced == 0)
-                          ? key_splits(p.B, p.Hq, p.H, p.Nq, p.N, std::min(sms, SPLIT_SIZING_SMS)) : 1;
-  const bool ragged = n_split > 1 || (!p.causal && !varlen && !fast && !two && mostly_empty_tiles(p));
-  const int fold = ragged ? (int)(p.Hq / p.H) : 1;
+  const AttnForm form = choose_form({p.B, p.Hq, p.H, p.Nq, p.N, p.causal, varlen ? p.Tq : 0, p.plan != nullptr, p.part != nullptr,
+                                     !p.no_fast_path && skip > 0.f, g_force_tiles_per_cta.load(std::memory_order_relaxed)}, sms);
+  const bool two = form.two, fast = form.fast, ragged = form.ragged;
+  const int n_split = form.splits, fold = form.fold;
   if (ragged) { p.Nq = p_in.Nq * fold; p.Hq = p.H; }
   const uint64_t bh = (uint64_t)(p.B * p.H), N_pad = (uint64_t)p.N_pad;
   const uint64_t bhq = (uint64_t)(p.B * p.Hq), Nq = (uint64_t)p.Nq;

@@ -381,6 +381,27 @@ int sage_attention_tiles_per_cta(int64_t B, int64_t Hq, int64_t Nq, int causal, 
   return sage::choose_tiles_per_cta((Nq + sage::TILE - 1) / sage::TILE, B * Hq, causal != 0, sm_count);
 }
 
+int sage_attention_form(int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int64_t packed_q, int causal,
+                        int plain, int sm_count, int form[4]) {
+  g_err[0] = 0;
+  const Dims d = {B, Hq, Hkv, Nq, Nk, sage::HD};
+  int rc = check_dims(d);
+  if (rc) return rc;
+  if (packed_q < 0 || sm_count < 1 || !form) return fail(SAGE_E_ARG, "sage_attention_form: bad argument");
+  // what attention_impl hands over with a workspace of sage_workspace_bytes_ex bytes
+  const Layout L = carve(d);
+  char room;
+  const Packed pk = {nullptr, nullptr, packed_q, 0, &room, L.vmean - L.qm};
+  const sage::AttnForm f = sage::choose_form(
+      {B, Hq, Hkv, Nq, Nk, causal ? 1 : 0, packed_q, packed_q > 0 && packed_plan(d, pk) != nullptr, L.total > L.base_total, !plain, 0},
+      sm_count);
+  form[0] = f.two ? 2 : 1;
+  form[1] = f.splits;
+  form[2] = f.fold;
+  form[3] = f.fast && f.splits == 1 ? 1 : 0;
+  return 4;
+}
+
 size_t sage_workspace_bytes(int64_t B, int64_t H, int64_t N) {
   if (B < 1 || H < 1 || N < 1) return 0;
   const Dims d = {B, H, H, N, N, sage::HD};

@@ -68,6 +68,25 @@ size_t prologue_ctrl_bytes(int64_t B, int64_t H, int64_t N);
 // Returns cudaSuccess or an error; `why` (if non-null) receives a static description on failure.
 cudaError_t launch_attention(const AttnParams& p, cudaStream_t st, const char** why);
 
+// How the attention kernel serves a call: what launch_attention launches, as host arithmetic.
+struct AttnShape {
+  int64_t B, Hq, H, Nq, N;     // batch, query heads, K/V heads, queries, keys (longest lengths of a packed batch)
+  int causal;
+  int64_t packed_q;            // packed batch: tokens of q; 0 for a fixed-length call
+  bool work_list;              // packed batch: it has a work list
+  bool scratch;                // the shares of a split call have room
+  bool tests;                  // the negligible-tile tests are wanted
+  int forced;                  // 1 or 2: that many query tiles per CTA (test hook), 0: free
+};
+struct AttnForm {
+  bool two;                    // two query tiles per CTA
+  bool fast;                   // kernels with the negligible-tile tests
+  bool ragged;                 // RAGGED or SPLIT kernels
+  int fold;                    // query heads that share a unit's query tiles
+  int splits;                  // shares of the key range (1: not split)
+};
+AttnForm choose_form(const AttnShape& c, int sms);
+
 // Scratch for the partial results of a call whose keys are split over CTAs (0: never split); sized
 // without a device at hand, for the largest SM count an sm_100 part has.
 constexpr int SPLIT_SIZING_SMS = 160;

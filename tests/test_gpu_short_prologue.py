@@ -22,6 +22,13 @@ def test_bytes_and_scales(b, h, n, smooth_k, dtype):
     pq = be.quant_qkv(q.cuda(), k.cuda(), v.cuda(), smooth_k=smooth_k)
     torch.cuda.synchronize()
     _check_against(pq, ref, n, smooth_k)
+    # Which form ran: the one-launch form leaves the number of its tiles in the work counter, the
+    # persistent quantiser has drawn that many, the fold items and one item more per CTA.
+    tiles = 3 * b * h * ((n + 127) // 128)
+    counter = pq["ctrl"].view(torch.int32)[4 * b * h + 2].item()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    short = n <= 16 * 128 and (tiles + 1) // 2 <= 5 * sms        # K and V tiles share a CTA, and Q tiles in twos
+    assert counter == tiles if short else counter > tiles
 
 
 @pytest.mark.parametrize("hq,hkv,nq,nk,d,lse,smooth_v", [

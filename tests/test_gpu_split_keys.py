@@ -9,6 +9,7 @@ import torch
 from oracle import ref_numerics as R
 from sageattention import _native
 from sageattention import b200_backend as be
+from test_call_forms import form
 
 pytestmark = pytest.mark.gpu
 
@@ -31,6 +32,8 @@ def _inputs(b, hq, hkv, nq, nk, d, dtype, layout="HND"):
 ])
 def test_split_keys(b, hq, hkv, nq, nk, d, dtype, layout, smooth_v):
     lib = _native.load()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert form(b, hq, hkv, nq, nk, sms=sms)[1] > 1             # the call does split
     q, k, v = _inputs(b, hq, hkv, nq, nk, d, dtype, layout)
     kw = dict(tensor_layout=layout, return_lse=True, smooth_v=smooth_v)
     out, lse = be.sage_call(q, k, v, **kw)
