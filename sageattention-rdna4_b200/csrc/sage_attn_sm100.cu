@@ -1257,10 +1257,15 @@ AttnForm choose_form(const AttnShape& c, int sms) {
   // 12.7 / 14.4; 2 x 24 x 1 000 x 1 000 39.4 / 45.5; but 48 x 2 048 x 2 048 (16 key tiles) 121 / 118.
   f.two = !short_loop && choose_tiles_per_cta((c.Nq + TILE - 1) / TILE, c.B * c.Hq, c.causal != 0, sms) == 2;
   if (c.forced != 0) f.two = (c.forced == 2);
-  // Packed batches: two tiles per CTA once there are about ten rounds of such CTAs, so that what is
-  // left over at the end (CTAs come longest first) does not weigh: 48 heads, 36 k tokens in eleven sequences of
-  // 512 .. 8 192 (46 rounds), whole call 4 369 us with one tile, 4 216 with two.
-  if (varlen) f.two = c.work_list && (c.forced ? c.forced == 2 : c.packed_q / (2 * TILE) * c.Hq >= 10 * (int64_t)sms);
+  // Packed batches: two tiles per CTA for long sequences only.  A sequence with an odd number of query
+  // tiles leaves half a CTA empty, and the one-tile kernels wait less often for P.V (PAIRED), so that two
+  // tiles gain little and lose much.  Two / one, whole call, 16 to 48 heads at ten rounds of CTAs and more:
+  // 8 192 tokens a sequence 0.96 to 1.00, 5 300 0.98 to 0.99, 6 000 1.00, 4 100 1.00 to 1.02, 3 100 1.03,
+  // 2 048 1.01, 300 1.25, 128 1.45 (the attention kernel alone 2.2); causal up to 1.07, and 1.00 at best.
+  if (varlen) {
+    const bool long_ones = c.packed_q >= 40 * TILE * c.B && c.packed_q / (2 * TILE) * c.Hq >= 10 * (int64_t)sms;
+    f.two = c.work_list && (c.forced ? c.forced == 2 : long_ones && !c.causal && !short_loop);
+  }
   // Neither a packed batch nor a loop over few key tiles takes the negligible-tile tests (most of such a
   // CTA's time is its start and end).
   f.fast = c.tests && !varlen && !short_loop;
