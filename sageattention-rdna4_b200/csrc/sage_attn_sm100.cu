@@ -1226,11 +1226,29 @@ int choose_tiles_per_cta(int64_t q_tiles, int64_t bhq, bool causal, int sms) {
 // longer calls, whose key tiles the negligible-tile tests may drop, on one pass.  2 x 8 K/V heads x
 // 4 x 4 query rows x 16 384 keys: 64 CTAs of 128 key tiles took 182 us, 256 of 8 with both passes
 // and the merge 35 us (whole call 267 -> 118 us).
+// The split form takes Q.K^T twice and two launches more, so it has to shorten the walk by enough.
+// Whole call, split / one pass, us; "rows" are the query rows of a K/V head:
+//   four shares and more pay at every size timed, least at 74 units x 32 tiles x 128 rows (119.0 / 123.9);
+//   three pay for up to 32 rows (98 x 32 tiles x 16 rows 129.5 / 133.8), whose CTAs do not slow each
+//     other down on an SM; with more rows while there is an SM for every share (49 x 24 x 128 rows 77.9 /
+//     82.8; 64 x 24 98.0 / 92.9) or the keys are many (80 x 48 x 96 rows 175 / 180, 96 x 96 x 128 rows
+//     352 / 360; but 96 x 32 x 128 rows 146.9 / 139.9);
+//   two pay for two softmax warps per CTA, which are slow alone (17 to 32 rows: 37 x 18 x 32 rows 58.4 / 61.3),
+//     while there is an SM for every share, and for up to 32 rows against very many keys (99 x 128 x 32 rows
+//     467 / 488, 110 x 256 x 4 rows 929 / 945); else they cost (100 x 16 x 128 rows 101.5 / 83.3, 100 x 64 x
+//     128 287.5 / 259.9, 128 x 16 x 4 95.2 / 89.6).
+// Keys of which 0.1 % are scaled x50, whose tiles one pass may skip, gain more by the same splits (64 units
+// x 128 tiles x 128 rows 323 / 385).
 int key_splits(int64_t B, int64_t Hq, int64_t H, int64_t Nq, int64_t Nk, int sms) {
-  const int64_t key_tiles = (Nk + TILE - 1) / TILE;
-  const int64_t units = B * H * ((Nq * (Hq / H) + TILE - 1) / TILE);
+  const int64_t key_tiles = (Nk + TILE - 1) / TILE, rows = Nq * (Hq / H);
+  const int64_t units = B * H * ((rows + TILE - 1) / TILE);
   if (Nq > TILE || key_tiles < 16 || units >= sms) return 1;
-  return (int)std::min<int64_t>(2 * sms / units, key_tiles / 8);
+  const int64_t n = std::min<int64_t>(2 * sms / units, key_tiles / 8);
+  const bool an_sm_each = n * units <= sms;
+  bool pays = n >= 4;
+  if (n == 3) pays = rows <= 32 || an_sm_each || key_tiles >= (rows <= 96 ? 48 : 96);
+  if (n == 2) pays = rows <= 16 ? key_tiles >= 256 : rows <= 32 && (an_sm_each || key_tiles >= 128);
+  return pays ? (int)n : 1;
 }
 size_t split_scratch_bytes(int64_t B, int64_t Hq, int64_t H, int64_t Nq, int64_t Nk) {
   const int n = key_splits(B, Hq, H, Nq, Nk, SPLIT_SIZING_SMS);

@@ -59,6 +59,51 @@ def test_packed_batches_without_a_work_list_take_one_tile():
     assert form(513, 96, 96, 8192, 8192, packed_q=513 * 8192)[0] == 1
 
 
+@pytest.mark.parametrize("units,tiles,rows,shares", [
+    # calls timed both ways on a 148-SM part: whole call, split / one pass over the keys, in us
+    (1, 32, 4, 4), (74, 32, 128, 4), (50, 32, 128, 4), (16, 128, 128, 16), (37, 40, 64, 5),      # all gain
+    (98, 32, 16, 3),          # 129.5 / 133.8
+    (80, 32, 32, 3),          # 119.0 / 129.1
+    (49, 24, 128, 3),         # 77.9 / 82.8
+    (64, 24, 128, 1),         # 98.0 / 92.9
+    (75, 32, 128, 1),         # 129.9 / 126.1
+    (96, 32, 128, 1),         # 146.9 / 139.9
+    (80, 48, 96, 3),          # 175.2 / 179.6
+    (96, 48, 128, 1),         # 197.8 / 195.5
+    (96, 96, 128, 3),         # 351.8 / 360.0
+    (128, 16, 4, 1),          # 95.2 / 89.6
+    (16, 16, 4, 1),           # 39.0 / 37.7
+    (100, 16, 128, 1),        # 101.5 / 83.3
+    (100, 64, 128, 1),        # 287.5 / 259.9
+    (147, 128, 128, 1),       # 684 / 636
+    (37, 18, 32, 2),          # 58.4 / 61.3
+    (147, 16, 32, 1),
+    (99, 128, 32, 2),         # 467.4 / 487.8
+    (110, 256, 4, 2),         # 929 / 945
+    (148, 256, 4, 1),         # a unit for every SM
+    (16, 15, 4, 1),
+])
+def test_shares_of_the_keys(units, tiles, rows, shares):
+    assert form(1, units, units, rows, tiles * 128)[1] == shares
+    if rows % 4 == 0:         # the rows of a K/V head count, whether they are queries or heads of its group
+        assert form(1, 4 * units, units, rows // 4, tiles * 128)[1] == shares
+
+
+def test_the_workspace_holds_the_shares_of_every_device():
+    """Its size is fixed without a device; no SM count up to the one it is sized for needs more."""
+    lib = _native.load()
+    offs = (ctypes.c_size_t * 13)()
+    for units in (1, 7, 36, 48, 49, 53, 54, 64, 74, 80, 96, 100, 120, 147, 159):
+        for nq in (1, 16, 17, 32, 33, 96, 97, 128):
+            for tiles in (16, 23, 24, 31, 32, 47, 48, 96, 128, 256):
+                nk = 128 * tiles - 5
+                assert lib.sage_workspace_layout_ex(1, units, units, nq, nk, offs) == 13
+                room = lib.sage_workspace_bytes_ex(1, units, units, nq, nk) - (offs[12] + units * 512)
+                for sms in (64, 100, 132, 144, 148, 152, 160, 200):
+                    n = form(1, units, units, nq, nk, sms=sms)[1]
+                    assert n == 1 or n * units * nq * 131 * 4 <= room, (units, nq, tiles, sms)
+
+
 def test_bad_arguments():
     out = (ctypes.c_int * 4)()
     f = _native.load().sage_attention_form

@@ -22,18 +22,22 @@ def _inputs(b, hq, hkv, nq, nk, d, dtype, layout="HND"):
     return tuple(t.transpose(1, 2).contiguous() for t in (q, k, v)) if layout == "NHD" else (q, k, v)
 
 
-@pytest.mark.parametrize("b,hq,hkv,nq,nk,d,dtype,layout,smooth_v", [
-    (1, 1, 1, 1, 2048, 128, torch.float16, "HND", False),      # one row, the shortest split key range
-    (2, 8, 2, 4, 16384, 128, torch.float16, "HND", False),     # folded heads, many shares
-    (1, 4, 1, 33, 2049, 128, torch.bfloat16, "NHD", False),    # folded rows in two tiles; one key in the last tile
-    (1, 12, 4, 128, 5000, 96, torch.bfloat16, "NHD", True),    # narrow heads, smooth_v, ragged shares
-    (3, 5, 5, 128, 4321, 64, torch.float16, "HND", True),
-    (1, 147, 147, 17, 2300, 128, torch.float16, "HND", False), # one unit short of the SM count
+@pytest.mark.parametrize("b,hq,hkv,nq,nk,d,dtype,layout,smooth_v,splits", [
+    (1, 1, 1, 1, 3072, 128, torch.float16, "HND", False, True),      # one row, the shortest key range that it splits
+    (2, 8, 2, 4, 16384, 128, torch.float16, "HND", False, True),     # folded heads, many shares
+    (1, 4, 1, 33, 3073, 128, torch.bfloat16, "NHD", False, True),    # folded rows in two tiles; one key in the last tile
+    (1, 12, 4, 128, 5000, 96, torch.bfloat16, "NHD", True, True),    # narrow heads, smooth_v, ragged shares
+    (3, 5, 5, 128, 4321, 64, torch.float16, "HND", True, True),
+    (1, 37, 37, 32, 2304, 128, torch.float16, "HND", False, True),   # two shares
+    (1, 98, 98, 17, 4100, 128, torch.bfloat16, "HND", False, True),  # three shares, two CTAs to an SM
+    (1, 1, 1, 1, 2048, 128, torch.float16, "HND", False, False),     # sizes at which one pass is faster
+    (1, 4, 1, 33, 2049, 128, torch.bfloat16, "NHD", False, False),
+    (1, 147, 147, 17, 2300, 128, torch.float16, "HND", False, False),
 ])
-def test_split_keys(b, hq, hkv, nq, nk, d, dtype, layout, smooth_v):
+def test_split_keys(b, hq, hkv, nq, nk, d, dtype, layout, smooth_v, splits):
     lib = _native.load()
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert form(b, hq, hkv, nq, nk, sms=sms)[1] > 1             # the call does split
+    assert (form(b, hq, hkv, nq, nk, sms=sms)[1] > 1) == splits
     q, k, v = _inputs(b, hq, hkv, nq, nk, d, dtype, layout)
     kw = dict(tensor_layout=layout, return_lse=True, smooth_v=smooth_v)
     out, lse = be.sage_call(q, k, v, **kw)
