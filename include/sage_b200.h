@@ -86,7 +86,8 @@ size_t sage_prologue_ctrl_bytes(int64_t B, int64_t H, int64_t N);
  * Alignment: q, k, v, q8, k8, v8t, sk, sv, svp and ctrl (and vmean of sage_prologue_ex) are read or
  * written with 16-byte vector accesses and must be 16-byte aligned; a misaligned one is refused
  * with SAGE_E_ARG before anything is launched.  sq, s_fold, mean and qm need 4-byte alignment.
- * Three kernel launches (a one-block kernel that clears the control words, mean, quantise). */
+ * Three kernel launches (a one-block kernel that clears the control words, mean, quantise), or one of
+ * clusters for short calls (up to 2 048 keys, about two and a half rounds of CTAs); the same bytes. */
 int sage_prologue(const void* q, const void* k, const void* v,
                   void* q8, float* sq, void* k8, float* sk, void* v8t, float* sv, float* svp,
                   float* s_fold, float* mean, void* ctrl,
@@ -234,7 +235,18 @@ int sage_attention(const void* q, const void* k, const void* v, void* out,
  *              given, V minus this mean is what gets quantised and the attention kernel adds the
  *              mean back to every output row (the softmax weights of a row sum to one)
  * Every size of K/V tensors (k8, sk, v8t, sv, svp, s_fold, mean, ctrl) is as for sage_prologue with
- * H = Hkv and N = Nk; q8 and sq are (B*Hq, Nq, 128) and (B*Hq, Nq). */
+ * H = Hkv and N = Nk; q8 and sq are (B*Hq, Nq, 128) and (B*Hq, Nq).
+ *
+ * What a result depends on.  A (batch, K/V head) unit and its query heads are computed alike whatever
+ * else the call holds, bit for bit, with one exception: a non-causal whole call (sage_attention and
+ * its variants) of few queries against many keys, in which few units leave SMs idle, splits every
+ * head's keys into shares and merges them.  P has the same e4m3 codes; the fp32 sums over the keys are
+ * taken in another order.  How many shares follows from B * Hkv, the SM count and whether the
+ * workspace has all of its sage_workspace_bytes_ex bytes, so that the same unit in a larger call, on
+ * another device, in a packed batch or through sage_attn_fwd_ex (none of the last two splits) may
+ * differ in the last bits: by at most 1e-5 of the result's 2-norm before it is rounded to 16 bits,
+ * which is then a step of the 16-bit format here and there, and 4e-6 of the largest value in the LSE.
+ * sage_attention_form tells whether a call splits. */
 int sage_prologue_ex(const void* q, const void* k, const void* v,
                      void* q8, float* sq, void* k8, float* sk, void* v8t, float* sv, float* svp,
                      float* s_fold, float* mean, float* qm, float* vmean, void* ctrl,
@@ -309,7 +321,9 @@ int sage_attn_fwd_reported(const void* q8, const float* sq, const void* k8, cons
  *   causal         every sequence must have as many keys as queries (max_q == max_k is checked;
  *                  the per-sequence equality is the caller's promise)
  * Each sequence is quantised on its own (its own K mean with smooth_k, its own S), exactly as if it
- * were passed alone to sage_attention_ex: the results are bit-identical to per-sequence calls.
+ * were passed alone to sage_attention_ex: the results are bit-identical to per-sequence calls, except
+ * to calls that split their keys (few queries against many keys, see sage_attention_ex; a packed batch
+ * never does), from which they differ by the order of fp32 sums.
  * A sequence without queries costs nothing; one with queries and no keys gets rows of zeros.
  * The arrays are not validated (that would need them on the host); the kernels clamp every start
  * and end to the packed token counts, so that no access leaves q, k, v or out whatever they hold.

@@ -59,6 +59,51 @@ def test_split_keys(b, hq, hkv, nq, nk, d, dtype, layout, smooth_v, splits):
     assert (lse - one_lse).abs().max().item() <= 4e-6 * one_lse.abs().max().item() + 4e-6
 
 
+def _close(out, one, dtype):
+    """The stated distance of two calls that split the keys differently (see the top of the file)."""
+    step = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7
+    out, one = out.float(), one.float()
+    assert ((out - one).abs() <= step * one.abs() + 1e-4 * one.std()).all()
+    assert R.rel_l1(out, one) <= step / 8
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_a_packed_batch_against_calls_that_split(dtype):
+    """A packed batch never splits: its sequences equal the unsplit calls bit for bit, and the calls
+    that a program would make, which split, up to the order of fp32 sums."""
+    lib = _native.load()
+    hq, hkv, nq, nk = 4, 2, (4, 128, 1, 60), (4200, 5000, 4097, 4500)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert all(form(1, hq, hkv, a, b, sms=sms)[1] > 1 for a, b in zip(nq, nk))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(sum(n), h, 128, generator=g, device="cuda").to(dtype) for n, h in ((nq, hq), (nk, hkv), (nk, hkv)))
+    cu = lambda n: torch.tensor([sum(n[:i]) for i in range(len(n) + 1)], dtype=torch.int32, device="cuda")
+    out = be.sage_call_varlen(q, k, v, cu(nq), cu(nk), max(nq), max(nk))
+    a = b = 0
+    for n, m in zip(nq, nk):
+        args = (q[None, a:a + n], k[None, b:b + m], v[None, b:b + m], "NHD")
+        lib.sage_debug_tiles_per_cta(1)                        # a forced shape never splits
+        try:
+            assert torch.equal(out[a:a + n], be.sage_call(*args)[0])
+        finally:
+            lib.sage_debug_tiles_per_cta(0)
+        _close(be.sage_call(*args)[0], out[a:a + n], dtype)
+        a, b = a + n, b + m
+
+
+def test_units_of_a_split_call_one_by_one():
+    """The number of shares follows from the number of (batch, K/V head) units, so a unit computed
+    alone agrees with the whole call up to the order of fp32 sums."""
+    b, hq, hkv, nq, nk = 2, 80, 40, 8, 6000
+    q, k, v = _inputs(b, hq, hkv, nq, nk, 128, torch.float16)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert form(b, hq, hkv, nq, nk, sms=sms)[1] != form(1, 2, 1, nq, nk, sms=sms)[1]
+    whole = be.sage_call(q, k, v)
+    for i, h in ((0, 0), (0, 39), (1, 17)):
+        one = be.sage_call(q[i:i + 1, 2 * h:2 * h + 2], k[i:i + 1, h:h + 1], v[i:i + 1, h:h + 1])
+        _close(one, whole[i:i + 1, 2 * h:2 * h + 2], torch.float16)
+
+
 def test_a_workspace_without_the_scratch_is_still_accepted():
     """The C entry point takes a workspace that only lacks the shares' scratch, and does not split."""
     lib = _native.load()
