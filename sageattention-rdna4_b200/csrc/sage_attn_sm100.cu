@@ -509,6 +509,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (lane == 0) {
         const int g = warp & 1, gb = BAR_PER_TILE * g;
         const int n_tiles = tiles_of(g);
+        // Tiles to load; only the second query tile's issuers load, and its range is the longer one.  (The
+        // 32 registers these warps have do not hold the state of the causal kernels with the tests: 12
+        // bytes spill with both counts, 4 with one; 48 x 8 771, bf16 925.8 / 922.1 us.  The query tile as a
+        // constant of the code leaves none, but four copies of the loops: 48 x 47 520 16.8 -> 22.2 ms.)
+        const int n_loads = FAST && CAUSAL ? n_tiles : n_load;
         const uint32_t n_live = FAST ? (uint32_t)live_warps(g) : 0u;
         bool ok = true;
         if (warp < 2) {
@@ -533,7 +538,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               tma_load_3d(base + OFF_Q + t * TILE_BYTES, &tm_q, bar(BAR_Q), 0, (q_tile0 + t) * TILE, bh);
           } else {
             ok = load_k(0);
-            if (ok && n_load > 1) ok = load_k(1);
+            if (ok && n_loads > 1) ok = load_k(1);
           }
           if (ok) ok = mbar_wait(bar(BAR_Q), 0, cta_abort, a.status, ST_TIMEOUT_MMA);
           for (int j = 0; ok && j < n_tiles; ++j) {
@@ -549,7 +554,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                            kmajor_sw128_desc(base + OFF_K + s * TILE_BYTES + 32 * k), IDESC_QK, k > 0);
             tc_commit(bar(BAR_KE + s));
             tc_commit(bar(BAR_SF + gb));
-            if (warp == 1 && j + 2 < n_load) ok = load_k(j + 2);
+            if (warp == 1 && j + 2 < n_loads) ok = load_k(j + 2);
           }
         } else {
           // ------------------------------- P.V issuers -----------------------------
@@ -562,7 +567,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             return true;
           };
           if (warp == 3) {
-            for (int j = 0; ok && j < L::V_STAGES && j < n_load; ++j) ok = load_v(j);
+            for (int j = 0; ok && j < L::V_STAGES && j < n_loads; ++j) ok = load_v(j);
           }
           for (int jj = 0; ok && jj < n_tiles; ++jj) {
             const int s = jj % L::V_STAGES;
@@ -586,7 +591,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                             (jj > 0 || k > 0) ? 1u : 0u);
             tc_commit(bar(BAR_VE + s));
             tc_commit(of_pair(BAR_PV, gb, jj));
-            if (warp == 3 && jj + L::V_STAGES < n_load) ok = load_v(jj + L::V_STAGES);
+            if (warp == 3 && jj + L::V_STAGES < n_loads) ok = load_v(jj + L::V_STAGES);
           }
         }
       }
@@ -685,12 +690,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int q_tile = q_tile0 + g;
       const int quarter = warp & 3;                         // TMEM lane quarter this warp may touch
       const int sub = ((warp - 4) >> 2) & 1;                // which 16 lanes of the quarter
-      const int r0 = lane >> 2, c = lane & 3;
+      const int r0 = lane >> 2;
+      int c = lane & 3;
       const int lane_base = 32 * quarter + 16 * sub;
       if (ROWS == WHOLE || ROWS == NARROW || lane_base < 16 * live_warps(g)) {
       const int n_tiles = tiles_of(g);
       const int rowA = lane_base + r0, rowB = rowA + 8;     // this thread's two query rows of the tile
-      const long long q_rowA = (long long)q_tile * TILE + rowA, q_rowB = q_rowA + 8;
+      long long q_rowA = (long long)q_tile * TILE + rowA, q_rowB = q_rowA + 8;
       const uint32_t t_s = tmem + ((uint32_t)lane_base << 16) + L::tmem_s(g);
       const uint32_t t_o = tmem + ((uint32_t)lane_base << 16) + L::tmem_o(g);
       // c_q = f32(f32(sm_scale * log2e) * sq); rows past N get 1 (their scores are all zero)
@@ -970,6 +976,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (FAST && a.skipped != nullptr && lane == 0 && n_skipped > 0) atomicAdd(a.skipped, (unsigned)n_skipped);
 
       // ------------------------------- epilogue -----------------------------------
+      if (NQ == 1 && FAST && CAUSAL && !INT8) {
+        // This thread's rows, worked out again: kept across the loop they spill 28 bytes (24 heads x 4 096
+        // keys with dominant ones 139.4 us, without the spills 132.7; 8 heads 74.7 / 71.3).
+        int t;
+        asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+        c = t & 3;
+        q_rowA = (long long)q_tile * TILE + 32 * ((t >> 5) & 3) + 16 * (((t >> 5) - 4) >> 2 & 1) + ((t & 31) >> 2);
+        q_rowB = q_rowA + 8;
+      }
       if (ROWS == SPLIT_MAX) {
         const size_t row0 = (size_t)share * gridDim.y * a.Nq + (size_t)bh * a.Nq;
         if (ok && c == 0 && q_rowA < a.Nq) a.part_max[row0 + q_rowA] = mA;

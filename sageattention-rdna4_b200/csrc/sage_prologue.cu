@@ -488,6 +488,7 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                      const __grid_constant__ CUtensorMap tm_v, const QuantArgs a) {
   extern __shared__ uint8_t qt_smem[];
   __shared__ int4 s_item[QT_STAGES];   // what the stage holds: {tensor (0 q, 1 k, 2 v, 3 a fold, -1 the end), head, tile, live tokens}
+  __shared__ int s_drawn;              // thread 0's next item (in a register it makes the int8 kernels spill)
   __shared__ int s_plan[VARLEN ? 4 * (PLAN_MAX_SEQS + 1) : 1];
   const uint32_t raw_addr = qt_smem_u32(qt_smem);
   const uint32_t base = (raw_addr + 127u) & ~127u;
@@ -592,7 +593,7 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   int drawn = 0;
   if (tid == 0) {
     for (int p = 0; p < QT_STAGES - 1; ++p) issue(p, draw());
-    drawn = draw();
+    s_drawn = draw();
   }
   __syncthreads();                     // s_item of the first stage, for a thread whose wait runs out too
 
@@ -600,8 +601,8 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int stage = (int)(n % QT_STAGES);
     const uint32_t parity = (n / QT_STAGES) & 1u;
     if (tid == 0) {                    // into the stage released by the previous item
-      issue((int)((n + QT_STAGES - 1) % QT_STAGES), drawn);
-      drawn = draw();                  // consumed one iteration later
+      issue((int)((n + QT_STAGES - 1) % QT_STAGES), s_drawn);
+      s_drawn = draw();                // consumed one iteration later
     }
     // bounded wait for this item's tile; a thread that gives up goes on to the barrier at the end of
     // the item, where all leave together
