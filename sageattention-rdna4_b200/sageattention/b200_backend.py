@@ -255,7 +255,8 @@ def _env_flag(name: str, default: bool) -> bool:
 # synchronisation: the result is picked up by a later call once its event has completed); a probe
 # that skipped less than PROBE_MIN_SHARE of the (warp, key tile) pairs sends the next PLAIN_CALLS
 # calls of that signature to the kernels without the tests, after which the next call probes
-# again.  Both sets of kernels give identical bits whenever no tile is skipped.  (Break-even,
+# again.  A call whose kernels make no tests (a short key loop, split keys) does not probe.  Both sets
+# of kernels give identical bits whenever no tile is skipped.  (Break-even,
 # measured at H=16, N=16384: with 23 % of the pairs skipped the two sets take the same time.)
 PROBE_MIN_SHARE = 0.2
 PLAIN_CALLS = 255
@@ -407,6 +408,14 @@ def check(device=None):
     st.raise_if_failed("check()")
 
 
+def _tests_apply(dev, b: int, hq: int, hkv: int, nq: int, nk: int, is_causal: bool) -> bool:
+    """Whether a call of this size, left to itself, runs on kernels with the negligible-tile tests."""
+    form = (ctypes.c_int * 4)()
+    rc = _native.load().sage_attention_form(b, hq, hkv, nq, nk, 0, 1 if is_causal else 0, 0,
+                                            torch.cuda.get_device_properties(dev).multi_processor_count, form)
+    return rc == 4 and form[3] != 0
+
+
 # Calls repeat with the same shapes and strides (a diffusion transformer issues the same attention
 # call thousands of times), and for sequences of a few hundred tokens the GPU work is shorter than
 # a careless host path.  A call signature that has passed `envelope_reason` once is remembered with
@@ -517,6 +526,9 @@ def sage_call(q, k, v, tensor_layout="HND", is_causal=False, sm_scale=None, smoo
         plain, probe = ad.plain_left.get(key, 0) > 0, False
     else:
         plain, probe = ad.decide(key) if _ADAPTIVE else (False, False)
+        if probe and not _tests_apply(dev, b, h, hkv, n, nk, is_causal):
+            ad.take_result(key, 0, 1)                # nothing to find out: such a call skips no tile
+            plain, probe = True, False
     if plain:
         qk_mode = -_native.SAGE_QK_NO_FAST_PATH if qk_mode < 0 else (qk_mode | _native.SAGE_QK_NO_FAST_PATH)
     args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 0 if lse is None else lse.data_ptr(),

@@ -160,3 +160,27 @@ def test_skipped_pairs_are_counted_and_steer_the_choice_of_kernels():
     finally:
         be._ADAPTIVE = saved
         be.clear_workspaces()
+
+
+@pytest.mark.parametrize("nq,nk,probes", [
+    (300, 1000, False),        # up to eight key tiles: no kernel tests them
+    (4, 8192, False),          # split keys: nor do the kernels of the shares
+    (300, 1100, True),
+])
+def test_only_calls_that_may_skip_tiles_probe(nq, nk, probes):
+    """A probe (a copy of the count and an event behind the call) is made where there is something to
+    find out; other calls take the kernels without the tests from the first one on."""
+    saved = be._ADAPTIVE
+    be._ADAPTIVE = True
+    try:
+        be.clear_workspaces()
+        q = torch.randn(1, 4, nq, 128, device="cuda").half()
+        k, v = (torch.randn(1, 4, nk, 128, device="cuda").half() for _ in range(2))
+        be.sage_call(q, k, v)
+        torch.cuda.synchronize()
+        st = be._state(q.device, torch.cuda.current_stream().cuda_stream, create=False)
+        assert (st.adaptive.probe is not None) == probes
+        assert any(n > 0 for n in st.adaptive.plain_left.values()) == (not probes)
+    finally:
+        be._ADAPTIVE = saved
+        be.clear_workspaces()
