@@ -428,12 +428,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int key_tiles = VARLEN ? (int)((Nk_live + TILE - 1) / TILE)
                         : SPLIT ? min((int)(a.N_pad / TILE) - k_tile0, a.split_tiles) : (int)(a.N_pad / TILE);
   if (SPLIT) Nk_live = a.N - (long long)k_tile0 * TILE;      // keys from the first one of this share on
-  // Softmax warps of query tile g that hold a row that exists (16 rows each; one at least, so that
-  // an empty second tile keeps its barriers turning).  The others stay out of the loop and of the
+  // Softmax warps of query tile g that take part: all eight, but in the RAGGED and SPLIT kernels only
+  // those that hold a row that exists (16 rows each).  The others stay out of the loop and of the
   // barriers' counts: their rows of P are never written and their rows of O never read.
   auto live_warps = [&](int g) {
     if (ROWS == WHOLE || ROWS == NARROW) return 8;
-    const long long rows = (VARLEN ? Nq_live : a.Nq) - (long long)(q_tile0 + g) * TILE;
+    const long long rows = a.Nq - (long long)(q_tile0 + g) * TILE;       // (never a packed batch)
     return (int)min(max((rows + 15) / 16, 1LL), 8LL);
   };
   auto tiles_of = [&](int g) { return CAUSAL ? min(q_tile0 + g + 1, key_tiles) : key_tiles; };
@@ -514,7 +514,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // bytes spill with both counts, 4 with one; 48 x 8 771, bf16 925.8 / 922.1 us.  The query tile as a
         // constant of the code leaves none, but four copies of the loops: 48 x 47 520 16.8 -> 22.2 ms.)
         const int n_loads = FAST && CAUSAL ? n_tiles : n_load;
-        const uint32_t n_live = FAST ? (uint32_t)live_warps(g) : 0u;
         bool ok = true;
         if (warp < 2) {
           // ------------------------------- Q.K^T issuers ---------------------------
@@ -579,7 +578,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               volatile uint32_t* cnt = misc + 4 + 2 * g + (jj & 1);
               const uint32_t c8 = *cnt;
               if (c8 != 0u) *cnt = 0u;
-              all_zero = (c8 == n_live);
+              all_zero = (c8 == 8u);
             }
             tc_fence_after();
             if (!all_zero)
@@ -629,7 +628,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int g = 0;
       const int gb = BAR_PER_TILE * g;
       const int n_tiles = tiles_of(g);
-      const uint32_t n_live = FAST ? (uint32_t)live_warps(g) : 0u;
       if (lane == 0) {
         constexpr uint32_t IDESC_QK = INT8 ? IDESC_I8 : IDESC_F8;
         bool ok = mbar_wait(bar(BAR_Q), 0, cta_abort, a.status, ST_TIMEOUT_MMA);
@@ -653,7 +651,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (ok) ok = mbar_wait(of_pair(BAR_PF, gb, jj), pair_parity(jj), cta_abort, a.status, ST_TIMEOUT_MMA);
             if (!ok) break;
             // FAST kernels: a warp that skips a tile counts itself before it arrives at the P
-            // barrier.  When all live warps of the query tile did, P(jj) is all zeros and the
+            // barrier.  When all eight warps of the query tile did, P(jj) is all zeros and the
             // product is not issued; the two commits still release the V stage and complete the
             // P.V barrier (the first tile is never skipped, so the accumulator is initialised).
             bool all_zero = false;
@@ -661,7 +659,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               volatile uint32_t* cnt = misc + 4 + 2 * g + (jj & 1);
               const uint32_t c8 = *cnt;
               if (c8 != 0u) *cnt = 0u;
-              all_zero = (c8 == n_live);
+              all_zero = (c8 == 8u);
             }
             tc_fence_after();
             if (!all_zero)
