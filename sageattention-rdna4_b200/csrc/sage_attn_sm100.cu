@@ -1288,14 +1288,22 @@ AttnForm choose_form(const AttnShape& c, int sms) {
   // 12.7 / 14.4; 2 x 24 x 1 000 x 1 000 39.4 / 45.5; but 48 x 2 048 x 2 048 (16 key tiles) 121 / 118.
   f.two = !short_loop && choose_tiles_per_cta((c.Nq + TILE - 1) / TILE, c.B * c.Hq, c.causal != 0, sms) == 2;
   if (c.forced != 0) f.two = (c.forced == 2);
-  // Packed batches: two tiles per CTA for long sequences only.  A sequence with an odd number of query
-  // tiles leaves half a CTA empty, and the one-tile kernels wait less often for P.V (PAIRED), so that two
-  // tiles gain little and lose much.  Two / one, whole call, 16 to 48 heads at ten rounds of CTAs and more:
-  // 8 192 tokens a sequence 0.96 to 1.00, 5 300 0.98 to 0.99, 6 000 1.00, 4 100 1.00 to 1.02, 3 100 1.03,
-  // 2 048 1.01, 300 1.25, 128 1.45 (the attention kernel alone 2.2); causal up to 1.07, and 1.00 at best.
+  // Packed batches: two tiles per CTA for long sequences, once there are ten rounds of such CTAs.  A
+  // sequence with an odd number of query tiles leaves half a CTA empty, which takes as long as a full
+  // one: at most one tile in 36 may be such a half (one for every other sequence is expected,
+  // and known if all have the longest length), and the shape needs long loops to win at all.  Two / one, whole
+  // call, each side run for a quarter of a second at a time, fp16: 2 x 8 192 tokens, 48 heads 0.958;
+  // eleven of 512 to 8 192 0.979 (bursts with pauses between them 1.002), sixteen of 2 330 on average
+  // 0.980 (1.005); 8 x 2 048 0.988 (1.015);
+  // sixteen of 1 436 on average 0.993 (1.027); 8 x 3 100 (25 tiles each) 1.003 (1.030); sixteen of 559
+  // 1.062; 128 x 300 1.25; 64 x 128 1.45.  Causal, where half as many key tiles go to a query tile: eleven of
+  // 512 to 8 192 1.021, four of 4 198 on average 1.001, 2 x 8 192 0.985.
   if (varlen) {
-    const bool long_ones = c.packed_q >= 40 * TILE * c.B && c.packed_q / (2 * TILE) * c.Hq >= 10 * (int64_t)sms;
-    f.two = c.work_list && (c.forced ? c.forced == 2 : long_ones && !c.causal && !short_loop);
+    const int64_t longest = (c.Nq + TILE - 1) / TILE;                     // all in query tiles
+    const bool equal = c.packed_q >= c.B * c.Nq;
+    const int64_t tiles = equal ? c.B * longest : c.packed_q / TILE + c.B / 2, halves = equal ? c.B * (longest & 1) : c.B / 2;
+    const bool pays = tiles >= (c.causal ? 64 : 18) * c.B && 36 * halves <= tiles && c.packed_q / (2 * TILE) * c.Hq >= 10 * (int64_t)sms;
+    f.two = c.work_list && (c.forced ? c.forced == 2 : pays && !short_loop);
   }
   // Neither a packed batch nor a loop over few key tiles takes the negligible-tile tests (most of such a
   // CTA's time is its start and end).

@@ -41,14 +41,20 @@ def test_negligible_tile_tests():
     (128, 300, 128 * 300, 20, 0, 300, 1),            # 603 / 754
     (32, 512, 32 * 512, 46, 0, 512, 1),              # 491 / 532
     (16, 1024, 16 * 1024, 46, 0, 1024, 1),           # 644 / 680
-    (8, 2048, 8 * 2048, 96, 0, 2048, 1),             # 2002 / 2037
-    (8, 3100, 8 * 3100, 48, 0, 3100, 1),             # 2139 / 2208
-    (11, 8192, 36124, 48, 0, 8192, 1),               # 4152 / 4152
-    (5, 4100, 5 * 4100, 37, 0, 4100, 1),             # 1707 / 1732
-    (2, 8192, 2 * 8192, 48, 0, 8192, 2),             # 3066 / 2992
-    (5, 8192, 26705, 32, 0, 8192, 2),                # 2580 / 2554
+    (12, 1200, 12 * 1200, 53, 0, 1200, 1),           # 789 / 830
+    (16, 2000, 8944, 96, 0, 2000, 1),                # 887 / 940: ragged, 559 tokens on average
+    (8, 3100, 8 * 3100, 48, 0, 3100, 1),             # 2280 / 2283: 25 tiles each
+    (6, 3300, 6 * 3300, 40, 0, 3300, 2),             # 1554 / 1521: 26 tiles each
+    (11, 8192, 36124, 48, 0, 8192, 2),               # 4364 / 4276
+    (8, 6000, 22496, 48, 0, 6000, 2),                # 2826 / 2783
+    (16, 8192, 37280, 48, 0, 8192, 2),               # 3880 / 3802
+    (16, 4000, 22976, 48, 0, 4000, 1),               # 1730 / 1718, 1648 / 1694 in bursts: ragged, 1 436 on average
+    (2, 8192, 2 * 8192, 48, 0, 8192, 2),             # 3155 / 3025
+    (5, 8192, 26705, 32, 0, 8192, 2),                # 2682 / 2616
     (3, 8192, 3 * 8192, 8, 0, 8192, 1),              # 792 / 831: five rounds
-    (2, 8192, 2 * 8192, 48, 1, 8192, 1),             # 1754 / 1778
+    (11, 8192, 36124, 48, 1, 8192, 1),               # 2674 / 2723
+    (4, 8192, 16792, 48, 1, 8192, 1),                # 1697 / 1696
+    (2, 8192, 2 * 8192, 48, 1, 8192, 2),             # 1837 / 1810
     (2, 8192, 2 * 8192, 48, 0, 1024, 1),             # short key loops take one tile as in every other call
 ])
 def test_packed_batches(n_seq, longest, tokens, heads, causal, keys, tiles):
@@ -56,6 +62,7 @@ def test_packed_batches(n_seq, longest, tokens, heads, causal, keys, tiles):
 
 
 def test_packed_batches_without_a_work_list_take_one_tile():
+    assert form(512, 96, 96, 8192, 8192, packed_q=512 * 8192)[0] == 2
     assert form(513, 96, 96, 8192, 8192, packed_q=513 * 8192)[0] == 1
 
 
