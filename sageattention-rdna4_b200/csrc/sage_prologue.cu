@@ -120,7 +120,7 @@ kmean_kernel(const MeanOf<T> of_k, const MeanOf<T> of_v, long long N, long long 
   __shared__ double red[16][HD];
   __shared__ int s_last;
   wait_for_predecessor();            // the cleared arrival counters
-  allow_successor();                 // one wave: every CTA of this grid is resident
+  allow_successor();                 // (one wave, but for packed batches and for K and V together)
   const int tid = threadIdx.x, c = tid & 15, r = tid >> 4;
   const int split = blockIdx.x, bh = blockIdx.y;
   const long long b = bh / H, h = bh - b * H;
@@ -590,7 +590,6 @@ quant_qkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   };
 
   __syncthreads();
-  int drawn = 0;
   if (tid == 0) {
     for (int p = 0; p < QT_STAGES - 1; ++p) issue(p, draw());
     s_drawn = draw();
