@@ -157,7 +157,8 @@ int sage_attn_fwd(const void* q8, const float* sq, const void* k8, const float* 
  * is how a host learns of a device-side failure without waiting for every call; the reference
  * raises for such failures only in strict mode and otherwise falls back
  * (sageattention/sk1_backend/__init__.py:1022-1027,1114-1123).  Status bits: 1 TMA producer,
- * 2 MMA issuer, 4 softmax warp of the attention kernel; 8 tile load of the prologue. */
+ * 2 MMA issuer, 4 softmax warp of the attention kernel; 8 tile load of the prologue; 0x100 (see
+ * sage_attention_reported) is set beside them once the failure has been written to a host word. */
 int sage_status_mirror(const int32_t* status_dev, int32_t* status_host, int words, void* stream);
 
 /* Test hook (one process-wide atomic word): the attention kernel has two shapes, one or two
